@@ -713,7 +713,7 @@ rak_status run_resident(rak_ctx *ctx, rak_graph *gr, const uint32_t *q, const ui
   return RAK_OK;
 }
 
-rak_status modularity_dev(rak_ctx *ctx, const void *off, bool off64, const uint32_t *tgt, const float *wt, int64_t n,
+rak_status modularity_dev(rak_ctx *ctx, const void *off, bool off64, const uint32_t *tgt, const float *wt, int64_t n, int64_t m,
                           const uint32_t *labels, Tracker *tr, double *q) {
   DevBuf ctot, sums;
   RAK_TRY(ctx, ctot.alloc(size_t(std::max<int64_t>(n, 1)) * 8, tr));
@@ -721,7 +721,7 @@ rak_status modularity_dev(rak_ctx *ctx, const void *off, bool off64, const uint3
   RAK_TRY(ctx, cudaMemsetAsync(ctot.p, 0, ctot.bytes, ctx->stream));
   RAK_TRY(ctx, cudaMemsetAsync(sums.p, 0, sums.bytes, ctx->stream));
   double h[4] = {0, 0, 0, 0};
-  if (n > 0) RAK_TRY(ctx, rak::launch_modularity(off, off64, tgt, wt, n, labels, ctot.as<double>(), sums.as<double>(), ctx->stream));
+  if (n > 0) RAK_TRY(ctx, rak::launch_modularity(off, off64, tgt, wt, n, m, labels, ctot.as<double>(), sums.as<double>(), ctx->stream));
   RAK_TRY(ctx, cudaMemcpyAsync(h, sums.p, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
   RAK_TRY(ctx, cudaStreamSynchronize(ctx->stream));
   if (h[3] > 0) { set_err(ctx, "membership holds labels >= n"); return RAK_ERR_INVALID_ARGUMENT; }
@@ -868,7 +868,7 @@ rak_status rak_graph_run(rak_ctx *ctx, rak_graph *gr, const uint32_t *q, const r
   rr->modularity = std::numeric_limits<double>::quiet_NaN();
   RAK_CHECK(run_resident(ctx, gr, q, o ? o->initial_flags : nullptr, r, membership, &tr, rr));
   if (r.modularity)
-    RAK_CHECK(modularity_dev(ctx, gr->off, gr->off64, gr->tgt, gr->wt, gr->n, membership, &tr, &rr->modularity));
+    RAK_CHECK(modularity_dev(ctx, gr->off, gr->off64, gr->tgt, gr->wt, gr->n, gr->m, membership, &tr, &rr->modularity));
   rr->peak_device_bytes = tr.peak + size_t(gr->n) * 4;
   return RAK_OK;
 }
@@ -897,7 +897,7 @@ rak_status rak_lowmem_cuda(rak_ctx *ctx, const rak_csr *g, const uint32_t *q, co
   rr->h2d_ms = gr->h2d_ms;
   if (g->location == RAK_DEVICE) {
     RAK_CHECK(run_resident(ctx, gr, q, flags, r, membership, &tr, rr));
-    if (r.modularity) RAK_CHECK(modularity_dev(ctx, gr->off, gr->off64, gr->tgt, gr->wt, n, membership, &tr, &rr->modularity));
+    if (r.modularity) RAK_CHECK(modularity_dev(ctx, gr->off, gr->off64, gr->tgt, gr->wt, n, gr->m, membership, &tr, &rr->modularity));
     rr->peak_device_bytes = tr.peak;
     return RAK_OK;
   }
@@ -917,7 +917,7 @@ rak_status rak_lowmem_cuda(rak_ctx *ctx, const rak_csr *g, const uint32_t *q, co
   RAK_TRY(ctx, cudaStreamSynchronize(ctx->stream));
   rr->h2d_ms += ev.ms(0, 1);
   RAK_CHECK(run_resident(ctx, gr, qd.as<uint32_t>(), fd.as<uint8_t>(), r, labels.as<uint32_t>(), &tr, rr));
-  if (r.modularity) RAK_CHECK(modularity_dev(ctx, gr->off, gr->off64, gr->tgt, gr->wt, n, labels.as<uint32_t>(), &tr, &rr->modularity));
+  if (r.modularity) RAK_CHECK(modularity_dev(ctx, gr->off, gr->off64, gr->tgt, gr->wt, n, gr->m, labels.as<uint32_t>(), &tr, &rr->modularity));
   cudaEventRecord(ev.e[2], ctx->stream);
   RAK_TRY(ctx, cudaMemcpyAsync(membership, labels.p, size_t(n) * 4, cudaMemcpyDeviceToHost, ctx->stream));
   cudaEventRecord(ev.e[3], ctx->stream);
@@ -998,7 +998,7 @@ rak_status rak_modularity_f64(rak_ctx *ctx, const rak_csr *g, const uint32_t *me
     RAK_TRY(ctx, cudaMemcpyAsync(&hbad, bad.p, 4, cudaMemcpyDeviceToHost, ctx->stream));
     RAK_TRY(ctx, cudaStreamSynchronize(ctx->stream));
     if (hbad) { set_err(ctx, "invalid CSR (device check)"); return RAK_ERR_INVALID_CSR; }
-    return modularity_dev(ctx, g->offsets, g->offset_bits == 64, g->targets, g->weights, g->n, membership, nullptr, q);
+    return modularity_dev(ctx, g->offsets, g->offset_bits == 64, g->targets, g->weights, g->n, g->m, membership, nullptr, q);
   }
   if (rak_csr_validate_host(g) != RAK_OK) { set_err(ctx, "invalid CSR (host check)"); return RAK_ERR_INVALID_CSR; }
   const int64_t n = g->n, m = g->m;
@@ -1012,7 +1012,7 @@ rak_status rak_modularity_f64(rak_ctx *ctx, const rak_csr *g, const uint32_t *me
   if (m > 0) RAK_TRY(ctx, cudaMemcpyAsync(tgt.p, g->targets, size_t(m) * 4, cudaMemcpyHostToDevice, ctx->stream));
   if (g->weights && m > 0) RAK_TRY(ctx, cudaMemcpyAsync(wt.p, g->weights, size_t(m) * 4, cudaMemcpyHostToDevice, ctx->stream));
   if (n > 0) RAK_TRY(ctx, cudaMemcpyAsync(lab.p, membership, size_t(n) * 4, cudaMemcpyHostToDevice, ctx->stream));
-  return modularity_dev(ctx, off.p, g->offset_bits == 64, tgt.as<uint32_t>(), wt.as<float>(), n, lab.as<uint32_t>(), nullptr, q);
+  return modularity_dev(ctx, off.p, g->offset_bits == 64, tgt.as<uint32_t>(), wt.as<float>(), n, m, lab.as<uint32_t>(), nullptr, q);
 }
 
 rak_status rak_gen_rmat_device(rak_ctx *ctx, int scale, double edge_factor, double a, double b, double c,

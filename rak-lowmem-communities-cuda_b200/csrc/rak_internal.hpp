@@ -216,7 +216,7 @@ cudaError_t launch_labels_to_ids(uint32_t *m, const uint32_t *ks, int64_t n, cud
 cudaError_t launch_hub_degrees(const void *off, bool off64, const uint32_t *order, int64_t nhub,
                                int64_t *deg, cudaStream_t st);
 cudaError_t launch_modularity(const void *off, bool off64, const uint32_t *tgt, const float *wt,
-                              int64_t n, const uint32_t *labels, double *ctot, double *sums,
+                              int64_t n, int64_t m, const uint32_t *labels, double *ctot, double *sums,
                               cudaStream_t st);
 
 // Batches of graphs (rak_kernels.cu).

@@ -340,7 +340,7 @@ extern "C" rak_status rak_lowmem_cuda_noalloc(int device, void *stream, const ra
     double hm[4] = {0, 0, 0, 0};
     NA_TRY(cudaMemsetAsync(ctot, 0, size_t(n) * 8, st));
     NA_TRY(cudaMemsetAsync(sums, 0, 4 * 8, st));
-    NA_TRY(launch_modularity(g->offsets, off64, g->targets, g->weights, n, membership, ctot, sums, st));
+    NA_TRY(launch_modularity(g->offsets, off64, g->targets, g->weights, n, g->m, membership, ctot, sums, st));
     NA_TRY(cudaMemcpyAsync(hm, sums, sizeof(hm), cudaMemcpyDeviceToHost, st));
     NA_TRY(cudaStreamSynchronize(st));
     if (hm[3] > 0) return RAK_ERR_INVALID_ARGUMENT;  // labels >= n (from q) are not vertex ids
