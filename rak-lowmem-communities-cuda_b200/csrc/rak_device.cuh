@@ -39,39 +39,77 @@ __device__ __forceinline__ void sk_clear(Sketch<S> &s, uint32_t d = NONE) {
 // Weighted Misra-Gries accumulate with the reference CPU rule (inc/rakLowmem.hxx:63-89): add x to
 // every slot keyed c; otherwise the LAST zero-weight slot takes (c, x); otherwise every weight
 // drops by x, clamped at zero. Only adds, subtracts and max: bit-identical to the CPU.
-// Hits (the common case once labels settle) leave early; the miss path runs only when needed.
-#ifndef RAK_MG_MINFIRST
-#define RAK_MG_MINFIRST 0
-#endif
+// Hits (the common case once labels settle) leave early; the miss path runs only when needed. Its
+// slot search carries "no free slot seen yet" from the last slot down, so each slot costs one test
+// and two conditional moves.
 template <int S>
 __device__ __forceinline__ void mg_acc(Sketch<S> &s, uint32_t c, float x) {
   bool hit = false;
 #pragma unroll
-  for (int i = 0; i < S; ++i)
-    if (s.k[i] == c) { s.w[i] = __fadd_rn(s.w[i], x); hit = true; }
-  if (hit) return;
-#if RAK_MG_MINFIRST
-  // every weight positive: no free slot, the decrement follows (same outcome as the search below)
-  float mn = s.w[0];
-#pragma unroll
-  for (int i = 1; i < S; ++i) mn = fminf(mn, s.w[i]);
-  if (mn > 0.0f) {
-#pragma unroll
-    for (int i = 0; i < S; ++i) s.w[i] = fmaxf(__fsub_rn(s.w[i], x), 0.0f);
-    return;
+  for (int i = 0; i < S; ++i) {
+    const bool h = s.k[i] == c;
+    if (h) s.w[i] = __fadd_rn(s.w[i], x);
+    hit |= h;
   }
-#endif
-  int f = -1;
+  if (hit) return;
+  bool full = true;
 #pragma unroll
-  for (int i = 0; i < S; ++i)
-    if (s.w[i] == 0.0f) f = i;
-  if (f >= 0) {
-#pragma unroll
-    for (int i = 0; i < S; ++i)
-      if (i == f) { s.k[i] = c; s.w[i] = x; }
-  } else {
+  for (int i = S - 1; i >= 0; --i) {
+    const bool take = full && s.w[i] == 0.0f;
+    if (take) { s.k[i] = c; s.w[i] = x; }
+    full = full && !take;
+  }
+  if (full) {
 #pragma unroll
     for (int i = 0; i < S; ++i) s.w[i] = fmaxf(__fsub_rn(s.w[i], x), 0.0f);
+  }
+}
+
+// The same accumulate for unit weights: weights are whole numbers, held as 32-bit integers above a
+// common base. With no free slot every weight is at least 1, so "every weight drops by 1, clamped at
+// zero" is the base rising by 1 -- one add instead of a subtract and a maximum per slot -- and a free
+// slot is one whose weight equals the base. Equal to the float form while weights stay below 2^24
+// (the callers bound the edges of one sketch).
+template <int S>
+struct UnitSketch {
+  uint32_t k[S];
+  uint32_t w[S];
+  uint32_t base;
+};
+template <int S>
+__device__ __forceinline__ void unit_clear(UnitSketch<S> &s) {
+#pragma unroll
+  for (int i = 0; i < S; ++i) { s.k[i] = NONE; s.w[i] = 0u; }
+  s.base = 0u;
+}
+template <int S>
+__device__ __forceinline__ void unit_acc(UnitSketch<S> &s, uint32_t c) {
+  bool hit = false;
+#pragma unroll
+  for (int i = 0; i < S; ++i) {
+    const bool h = s.k[i] == c;
+    if (h) s.w[i] += 1u;
+    hit |= h;
+  }
+  if (hit) return;
+  bool full = true;
+#pragma unroll
+  for (int i = S - 1; i >= 0; --i) {
+    const bool take = full && s.w[i] == s.base;
+    if (take) { s.k[i] = c; s.w[i] = s.base + 1u; }
+    full = full && !take;
+  }
+  if (full) s.base += 1u;
+}
+// The weights as floats. ORDER: only their order is needed (the sketch goes straight to the argmax), so
+// the whole numbers keep their bits -- small floats in the same order, zero at zero -- and the
+// integer-to-float conversions, a quarter-rate instruction each, are saved.
+template <int S, bool ORDER>
+__device__ __forceinline__ void unit_to_sketch(const UnitSketch<S> &u, Sketch<S> &s) {
+#pragma unroll
+  for (int i = 0; i < S; ++i) {
+    s.k[i] = u.k[i];
+    s.w[i] = ORDER ? __uint_as_float(u.w[i] - u.base) : float(u.w[i] - u.base);
   }
 }
 

@@ -20,14 +20,14 @@
 #include "rak_device.cuh"
 #include "rak_internal.hpp"
 
-// Edges loaded ahead per lane in the scan pipeline, and the resident blocks per SM the register
+// Edges per stage of the scan pipeline, and the resident blocks per SM the register
 // budget is sized for. Four blocks (64 registers; the asynchronous instantiations spill a few
 // hundred bytes) against three (80 registers), measured on B200 on renumbered resident graphs, one
 // box, runs alternated: R-MAT s27 100.5-100.7 vs 102.3-102.4 ms at lower clocks, s24 ef32 weighted
 // 30.2 vs 31.4 ms, 2D lattice 2^25 9.0 vs 9.8 ms (on the graphs as given, earlier, four blocks were
 // 1-5% slower): the loads in flight of the extra warps pay for the spills.
 #ifndef RAK_SCAN_BATCH
-#define RAK_SCAN_BATCH 4
+#define RAK_SCAN_BATCH 2
 #endif
 #ifndef RAK_MIN_BLOCKS
 #define RAK_MIN_BLOCKS 4
@@ -140,44 +140,76 @@ __device__ __forceinline__ float edge_w(const float *wt, int64_t e) {
   else return ld_weight(wt + e);
 }
 
-// Sequential sketch of edges e, e+st, ... < ee of u (self-loops skipped), in edge order.
-// Software-pipelined in batches of four: the next batch's targets and weights are loaded while
-// the current batch's labels are gathered and accumulated. Positions past the end are given the
-// target u itself, which the self-loop rule skips. Labels are read with plain loads: they change
-// during the launch.
-template <int S, bool UNIT, int RULE>
-__device__ __forceinline__ void scan_range(Sketch<S> &sk, uint32_t u, int64_t e, int64_t ee, int st,
-                                           const uint32_t *tgt, const float *wt, const uint32_t *vin,
-                                           uint32_t base) {
+// Sequential accumulation (acc) of edges e, e+st, ... < ee of u (self-loops skipped), in edge order.
+// Software-pipelined in three stages of two edges: while one stage's labels are accumulated, the next
+// stage's labels and the targets (and weights) of the one after are on their way. Positions past the
+// end are given the target u itself, which the self-loop rule skips. Labels are read with plain loads:
+// they change during the launch. Before (two stages of four edges, labels waited for) -> now, with the
+// whole-number sketch below, measured on B200: R-MAT scale 24 ef 16 11.3 -> 10.5 ms, scale 22 3.37 -> 3.15
+// ms, scale 20 2.86 -> 2.52 ms, scale 22 ef 32 weighted 9.7 -> 9.2 ms; lattice 2047x2049 1.13 -> 1.15 ms,
+// SBM 2 M vertices 1.29 -> 1.33 ms. Three edges a stage: scale 20 2.27 ms, lattice 1.19 ms.
+template <bool UNIT, class ACC>
+__device__ __forceinline__ void scan_edges(ACC &&acc, uint32_t u, int64_t e, int64_t ee, int st, const uint32_t *tgt,
+                                           const float *wt, const uint32_t *vin, uint32_t base) {
   constexpr int B = RAK_SCAN_BATCH;
-  uint32_t t[B];
-  float w[B];
+  // edges of this lane: a chain is at most hub_min / 32, hub_chunk / 32 or lane_max edges, so an int holds
+  // it, and 32-bit counts keep the 64-bit address arithmetic to one add per stage
+  int left = int((ee - e + st - 1) / st);
+  const uint32_t *tp = tgt + e;
+  const float *wp = UNIT ? nullptr : wt + e;
+  uint32_t t[B], t1[B], c[B];
+  float w[B], w1[B];
 #pragma unroll
   for (int j = 0; j < B; ++j) {
-    const int64_t x = e + int64_t(j) * st;
-    t[j] = x < ee ? base + ld_edge(tgt + x) : u;
-    w[j] = x < ee ? edge_w<UNIT>(wt, x) : 0.0f;
+    t[j] = j < left ? base + ld_edge(tp + j * st) : u;
+    w[j] = j < left ? edge_w<UNIT>(wp, j * st) : 0.0f;
+    t1[j] = B + j < left ? base + ld_edge(tp + (B + j) * st) : u;
+    w1[j] = B + j < left ? edge_w<UNIT>(wp, (B + j) * st) : 0.0f;
   }
-  while (e < ee) {
-    uint32_t c[B];
 #pragma unroll
-    for (int j = 0; j < B; ++j) c[j] = ld_label(vin + t[j]);
-    const int64_t en = e + int64_t(B) * st;
-    uint32_t t2[B];
+  for (int j = 0; j < B; ++j) c[j] = ld_label(vin + t[j]);
+  tp += 2 * B * st;
+  if constexpr (!UNIT) wp += 2 * B * st;
+  for (; left > 0; left -= B) {
+    uint32_t c1[B], t2[B];
     float w2[B];
 #pragma unroll
+    for (int j = 0; j < B; ++j) c1[j] = ld_label(vin + t1[j]);
+#pragma unroll
     for (int j = 0; j < B; ++j) {
-      const int64_t x = en + int64_t(j) * st;
-      t2[j] = x < ee ? base + ld_edge(tgt + x) : u;
-      w2[j] = x < ee ? edge_w<UNIT>(wt, x) : 0.0f;
+      t2[j] = 2 * B + j < left ? base + ld_edge(tp + j * st) : u;
+      w2[j] = 2 * B + j < left ? edge_w<UNIT>(wp, j * st) : 0.0f;
     }
 #pragma unroll
     for (int j = 0; j < B; ++j)
-      if (t[j] != u) sk_acc<S, RULE>(sk, c[j], w[j]);
+      if (t[j] != u) acc(c[j], w[j]);
 #pragma unroll
-    for (int j = 0; j < B; ++j) { t[j] = t2[j]; w[j] = w2[j]; }
-    e = en;
+    for (int j = 0; j < B; ++j) { t[j] = t1[j]; c[j] = c1[j]; w[j] = w1[j]; t1[j] = t2[j]; w1[j] = w2[j]; }
+    tp += B * st;
+    if constexpr (!UNIT) wp += B * st;
   }
+}
+
+// Unit weights under the CPU rules accumulate in whole numbers (UnitSketch) where a sketch, clear at
+// the start, sees at most 2^24 edges: about half the instructions of the float form on a miss.
+template <int S, bool UNIT, int RULE>
+__host__ __device__ constexpr bool unit_sketch() { return UNIT && S > 1 && RULE == RULE_CPU; }
+
+// ORDER: the sketch goes straight to the argmax, with no merge in between (one lane per vertex).
+template <int S, bool UNIT, int RULE, bool ORDER = false>
+__device__ __forceinline__ void scan_range(Sketch<S> &sk, uint32_t u, int64_t e, int64_t ee, int st,
+                                           const uint32_t *tgt, const float *wt, const uint32_t *vin,
+                                           uint32_t base) {
+  if constexpr (unit_sketch<S, UNIT, RULE>()) {
+    if (ee - e <= (int64_t(st) << 24)) {
+      UnitSketch<S> us;
+      unit_clear(us);
+      scan_edges<UNIT>([&](uint32_t c, float) { unit_acc(us, c); }, u, e, ee, st, tgt, wt, vin, base);
+      unit_to_sketch<S, ORDER>(us, sk);
+      return;
+    }
+  }
+  scan_edges<UNIT>([&](uint32_t c, float w) { sk_acc<S, RULE>(sk, c, w); }, u, e, ee, st, tgt, wt, vin, base);
 }
 
 // Neighbour marking reads a neighbour's flag before storing it when the launch asks for it
@@ -243,9 +275,9 @@ __device__ __forceinline__ bool lane_vec_ok(const uint32_t *tgt, const float *wt
   return ((reinterpret_cast<uintptr_t>(tgt) | (wt ? reinterpret_cast<uintptr_t>(wt) : 0)) & 15u) == 0;
 }
 
-template <int S, bool UNIT, int RULE>
-__device__ __forceinline__ void scan_lane(Sketch<S> &sk, uint32_t u, int64_t e, int64_t ee, const uint32_t *tgt,
-                                          const float *wt, const uint32_t *vin, uint32_t base) {
+template <bool UNIT, class ACC>
+__device__ __forceinline__ void scan_vectors(ACC &&acc, uint32_t u, int64_t e, int64_t ee, const uint32_t *tgt,
+                                             const float *wt, const uint32_t *vin, uint32_t base) {
   if (e >= ee) return;
   int64_t v = e >> 2;
   const int64_t vend = (ee + 3) >> 2;
@@ -266,7 +298,20 @@ __device__ __forceinline__ void scan_lane(Sketch<S> &sk, uint32_t u, int64_t e, 
     if (v + 1 < vend) load_vec4<UNIT>(v + 1, ee, tgt, wt, t4, w4);
 #pragma unroll
     for (int j = 0; j < 4; ++j)
-      if (t[j] != u) sk_acc<S, RULE>(sk, c[j], UNIT ? 1.0f : w[j]);
+      if (t[j] != u) acc(c[j], UNIT ? 1.0f : w[j]);
+  }
+}
+
+template <int S, bool UNIT, int RULE>
+__device__ __forceinline__ void scan_lane(Sketch<S> &sk, uint32_t u, int64_t e, int64_t ee, const uint32_t *tgt,
+                                          const float *wt, const uint32_t *vin, uint32_t base) {
+  if constexpr (unit_sketch<S, UNIT, RULE>()) {
+    UnitSketch<S> us;
+    unit_clear(us);
+    scan_vectors<UNIT>([&](uint32_t c, float) { unit_acc(us, c); }, u, e, ee, tgt, wt, vin, base);
+    unit_to_sketch<S, true>(us, sk);
+  } else {
+    scan_vectors<UNIT>([&](uint32_t c, float w) { sk_acc<S, RULE>(sk, c, w); }, u, e, ee, tgt, wt, vin, base);
   }
 }
 
@@ -466,7 +511,7 @@ template <int S, bool UNIT, int RULE>
 __device__ __forceinline__ void staged_scan(Sketch<S> &sk, StageCtx &sc, uint32_t u, int64_t eb, int64_t ee,
                                             const uint32_t *tgt, const float *wt, const uint32_t *vin, uint32_t base,
                                             RunState *rs, long long timeout_ns) {
-  constexpr int B = RAK_SCAN_BATCH;
+  constexpr int B = 4;
   const int lane = threadIdx.x & 31;
   // Copies cover [cs, ce): cs the first edge at a 16-byte aligned address at or after eb, ce the
   // last such boundary at or before ee. Tile k copies [cs + k*STG_TILE, min(cs + (k+1)*STG_TILE, ce));
@@ -666,7 +711,7 @@ __device__ __forceinline__ void lane_batch(const LpaArgs &a, const G_<O> &g, con
   sk_clear<S, RULE>(sk, d);
   const bool vec = lane_vec_ok(g.tgt, g.wt) && ee - eb >= RAK_VEC_MIN_DEG;
   if (vec) scan_lane<S, UNIT, RULE>(sk, u, eb, ee, g.tgt, g.wt, vin, base);
-  else scan_range<S, UNIT, RULE>(sk, u, eb, ee, 1, g.tgt, g.wt, vin, base);
+  else scan_range<S, UNIT, RULE, true>(sk, u, eb, ee, 1, g.tgt, g.wt, vin, base);
   if constexpr (MODE == MODE_SYNC && S > 1)
     if (a.rescan) rescan_range<S, UNIT>(sk, u, eb, ee, g.tgt, g.wt, vin, base);
   uint32_t c;
