@@ -232,6 +232,7 @@ struct RunState {
   unsigned int abort;       // set when any wait gives up
   unsigned int error;       // rak_status of the failure
   unsigned int iterations;  // iterations performed
+  unsigned long long asym;  // k_symmetry's sum: 0 for a symmetric graph
 };
 
 __device__ __forceinline__ unsigned long long global_ns() {

@@ -609,7 +609,7 @@ rak_status run_resident(rak_ctx *ctx, rak_graph *gr, const uint32_t *q, const ui
   if (tr) tr->add(b.bytes());
 
   rak::LpaArgs a{};
-  a.off = gr->off; a.tgt = gr->tgt; a.wt = gr->wt; a.n = n;
+  a.off = gr->off; a.tgt = gr->tgt; a.wt = gr->wt; a.n = n; a.m = gr->m;
   a.order = gr->order; a.rg = gr->rg;
   a.chunk_hub = gr->chunk_hub; a.hub_first = gr->hub_first; a.hub_chunk = gr->ly.hub_chunk; a.nchunks = gr->nchunks;
   a.vcom0 = vcom0; a.vcom1 = b.vcom1.as<uint32_t>(); a.aff0 = b.aff0.as<uint8_t>(); a.aff1 = b.aff1.as<uint8_t>();
@@ -619,6 +619,7 @@ rak_status run_resident(rak_ctx *ctx, rak_graph *gr, const uint32_t *q, const ui
   a.iters = r.iters; a.start_iter = r.start; a.tolerance = r.tol; a.pickless_step = r.pickless;
   a.check_on_pickless = r.check_on_pickless; a.rescan = r.rescan; a.mark_test = rak::mark_test_for(a.n, gr->m); a.gpu_rule = r.rule == 2; a.timeout_ns = r.timeout_ns; a.tie_until = r.tie_until; a.stage = r.stage; a.grid_cap = r.max_blocks;
   a.dense_moved_edges = rak::dense_threshold(r.mode, r.dense_pct, gr->m);
+  a.pull = rak::pull_for(r.mode, r.iters, gr->m); a.all_flags = flags == nullptr;
   if (renum) {
     a.off = gr->rn_off.p; a.tgt = gr->rn_tgt.as<uint32_t>(); a.wt = gr->wt ? gr->rn_wt.as<float>() : nullptr;
     a.order = gr->rn_ident.as<uint32_t>();
@@ -665,6 +666,7 @@ rak_status run_resident(rak_ctx *ctx, rak_graph *gr, const uint32_t *q, const ui
     cudaEventRecord(ev.e[1], st);
     if (!renum) RAK_TRY(ctx, rak::launch_init_flags(a.aff0, sync ? a.aff1 : nullptr, flags, n, st));
     cudaEventRecord(ev.e[2], st);
+    if (a.pull) RAK_TRY(ctx, rak::launch_symmetry(a.off, gr->off64, a.tgt, n, gr->m, nullptr, nullptr, b.rs.p, st));
     if (r.iters > 0) {
       int grid = 0;
       RAK_TRY(ctx, rak::launch_lpa(a, r.slots, r.mode, gr->off64, st, &grid));
@@ -958,7 +960,7 @@ rak_status rak_graph_step(rak_ctx *ctx, rak_graph *gr, const rak_options *o, int
   if (sync) RAK_TRY(ctx, cudaMemsetAsync(aff_next, 0, size_t(n), st));
   else if (aff_next != aff_prev) RAK_TRY(ctx, cudaMemcpyAsync(aff_next, aff_prev, size_t(n), cudaMemcpyDeviceToDevice, st));
   rak::LpaArgs a{};
-  a.off = gr->off; a.tgt = gr->tgt; a.wt = gr->wt; a.n = n;
+  a.off = gr->off; a.tgt = gr->tgt; a.wt = gr->wt; a.n = n; a.m = gr->m;
   a.order = gr->order; a.rg = gr->rg;
   a.chunk_hub = gr->chunk_hub; a.hub_first = gr->hub_first; a.hub_chunk = gr->ly.hub_chunk; a.nchunks = gr->nchunks;
   if (sync) {
@@ -1269,7 +1271,7 @@ rak_status batch_enqueue(rak_ctx *ctx, rak_batch *b, const uint32_t *q, const Re
   RAK_TRY(ctx, rak::launch_init_flags(rb.aff0.as<uint8_t>(), sync ? rb.aff1.as<uint8_t>() : nullptr, nullptr, n, st));
   if (r.iters > 0) {
     rak::LpaArgs a{};
-    a.off = gr->off; a.tgt = gr->tgt; a.wt = gr->wt; a.n = n;
+    a.off = gr->off; a.tgt = gr->tgt; a.wt = gr->wt; a.n = n; a.m = gr->m;
     a.order = gr->order; a.rg = gr->rg;
     a.chunk_hub = gr->chunk_hub; a.hub_first = gr->hub_first; a.hub_chunk = gr->ly.hub_chunk; a.nchunks = gr->nchunks;
     a.vcom0 = b->vcom0.as<uint32_t>(); a.vcom1 = v1; a.aff0 = rb.aff0.as<uint8_t>(); a.aff1 = sync ? rb.aff1.as<uint8_t>() : nullptr;
@@ -1281,6 +1283,8 @@ rak_status batch_enqueue(rak_ctx *ctx, rak_batch *b, const uint32_t *q, const Re
     a.running = b->running.as<unsigned int>(); a.ngraphs = G; a.grid_cap = grid_cap > 0 ? grid_cap : r.max_blocks;
     a.iters = r.iters; a.start_iter = r.start; a.tolerance = r.tol; a.pickless_step = r.pickless;
     a.check_on_pickless = r.check_on_pickless; a.rescan = r.rescan; a.mark_test = rak::mark_test_for_batch(a.n, gr->m, G); a.gpu_rule = r.rule == 2; a.timeout_ns = r.timeout_ns; a.tie_until = r.tie_until; a.stage = r.stage;
+    a.pull = rak::pull_for(r.mode, r.iters, gr->m); a.all_flags = 1;
+    if (a.pull) RAK_TRY(ctx, rak::launch_symmetry(gr->off, true, gr->tgt, n, gr->m, a.gid, a.vbase, rb.rs.p, st));
     int grid = 0;
     RAK_TRY(ctx, rak::launch_lpa(a, r.slots, r.mode, true, st, &grid, true));
   }

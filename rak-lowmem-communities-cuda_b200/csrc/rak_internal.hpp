@@ -83,6 +83,7 @@ __host__ __device__ inline int key_region(uint32_t key) { return key < 6 ? int(k
 
 struct RunStateHost {
   unsigned int bar, abort, error, iterations;
+  unsigned long long asym;
 };
 
 // Everything the persistent LPA kernel needs.
@@ -90,7 +91,7 @@ struct LpaArgs {
   const void *off;          // int32 or int64 offsets (template parameter of the kernel)
   const uint32_t *tgt;
   const float *wt;          // nullptr: unit weights
-  int64_t n;
+  int64_t n, m;
   const uint32_t *order;
   Regions rg;
   const uint32_t *chunk_hub;   // per chunk: index of its split vertex within region 0
@@ -129,7 +130,13 @@ struct LpaArgs {
   // asynchronous single graphs: an iteration marks no neighbours (and the next processes every
   // vertex) when the previous iteration's moved vertices hold at least this many edges; 0: never
   unsigned long long dense_moved_edges;
+  // synchronous modes: k_symmetry has run before the launch, so iterations may find their active set by
+  // looking for neighbours that moved (lpa_run); all_flags: every vertex starts affected
+  int pull, all_flags;
 };
+
+// Whether a run asks k_symmetry for that: it needs a second iteration to gain anything.
+inline int pull_for(int mode, int iters, int64_t m) { return mode != 0 && iters > 1 && m > 0 ? 1 : 0; }
 
 enum Mode { MODE_ASYNC = 0, MODE_SYNC = 1, MODE_SPLIT = 2 };
 
@@ -180,6 +187,11 @@ inline int mark_test_for(int64_t n, int64_t m) { return n >= (int64_t(1) << 22) 
 inline int mark_test_for_batch(int64_t n, int64_t m, int64_t graphs) {
   return graphs > 0 ? mark_test_for(n / graphs, m / graphs) : 0;
 }
+// Adds to rs->asym (RunState) a sum that is zero if every edge (u, v) has its reverse: each edge adds a
+// 64-bit hash of its unordered pair, positive from the smaller end, negative from the larger. gid, vbase:
+// the graphs of a batch (local targets), or null.
+cudaError_t launch_symmetry(const void *off, bool off64, const uint32_t *tgt, int64_t n, int64_t m, const uint32_t *gid,
+                            const int64_t *vbase, void *rs, cudaStream_t st);
 // Loads and resolves the kernel a run will launch (outside its timed region).
 cudaError_t prepare_lpa(int slots, int mode, bool off64, bool unit, bool batch, bool stage);
 

@@ -222,13 +222,10 @@ __device__ __forceinline__ int64_t row_at(const O *off, int64_t n, int64_t cost,
   return lo;
 }
 
-template <class O, bool UNIT>
-__global__ void __launch_bounds__(TPB) k_mod_edges(const O *off, const uint32_t *tgt, const float *wt, int64_t n, int64_t m,
-                                                   const uint32_t *labels, double *ctot, double *sums) {
-  constexpr int B = MOD_BATCH<UNIT>;
-  const int lane = threadIdx.x & 31;
-  const int64_t w = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5, nw = (int64_t(gridDim.x) * blockDim.x) >> 5;
-  // this warp's edges [e, e1): share w of the edges and rows laid end to end
+// Edges [e, *e1) of warp w of nw -- its share of the edges and rows laid end to end -- and the row of e.
+template <class O>
+__device__ __forceinline__ int64_t warp_edges(const O *off, int64_t n, int64_t m, int64_t w, int64_t nw, int64_t *e1,
+                                              int64_t *first_row) {
   const int64_t mo = int64_t(off[n]);
   const double share = double(m + MOD_ROW_COST * n) / double(nw);
   int64_t bound[2], row = 0;
@@ -239,8 +236,18 @@ __global__ void __launch_bounds__(TPB) k_mod_edges(const O *off, const uint32_t 
     const int64_t b = int64_t(off[row]) + (x - (int64_t(off[row]) + MOD_ROW_COST * row)), re = int64_t(off[row + 1]);
     bound[i] = w + i == nw ? mo : (b > re ? re : b);
   }
-  int64_t e = bound[0];
-  const int64_t e1 = bound[1] < mo ? bound[1] : mo;
+  *e1 = bound[1] < mo ? bound[1] : mo;
+  *first_row = row;
+  return bound[0];
+}
+
+template <class O, bool UNIT>
+__global__ void __launch_bounds__(TPB) k_mod_edges(const O *off, const uint32_t *tgt, const float *wt, int64_t n, int64_t m,
+                                                   const uint32_t *labels, double *ctot, double *sums) {
+  constexpr int B = MOD_BATCH<UNIT>;
+  const int lane = threadIdx.x & 31;
+  const int64_t w = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5, nw = (int64_t(gridDim.x) * blockDim.x) >> 5;
+  int64_t row, e1, e = warp_edges(off, n, m, w, nw, &e1, &row);
   double in_w = 0.0, hot_w = 0.0, tot_w = 0.0;
   unsigned long long in_n = 0, hot_n = 0;
   uint32_t hot = NONE;   // the label whose total this warp is keeping (all lanes agree)
@@ -379,6 +386,55 @@ __global__ void __launch_bounds__(TPB) k_mod_edges(const O *off, const uint32_t 
     if constexpr (UNIT) { if (blockIdx.x == 0) sums[1] = double(m); }
     else if (b != 0.0) atomicAdd(sums + 1, b);
   }
+}
+
+// launch_symmetry's sum. The edges are split over the warps as in k_mod_edges; the path is one stream of
+// the targets with a 64-bit mix per edge.
+constexpr int SYM_BATCH = 8;
+template <class O>
+__global__ void __launch_bounds__(TPB) k_symmetry(const O *off, const uint32_t *tgt, int64_t n, int64_t m,
+                                                  const uint32_t *gid, const int64_t *vbase, RunState *rs) {
+  const int lane = threadIdx.x & 31;
+  const int64_t w = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5, nw = (int64_t(gridDim.x) * blockDim.x) >> 5;
+  int64_t row, e1, e = warp_edges(off, n, m, w, nw, &e1, &row);
+  unsigned long long acc = 0;
+  for (int64_t ub = row; e < e1; ub += 32) {
+    const int64_t r = ub + lane;
+    const int64_t ob = int64_t(off[r < n ? r : n]), oe = int64_t(off[r < n ? r + 1 : n]);
+    const int64_t wend = __shfl_sync(FULL, oe, 31);
+    if (wend <= e) {
+      const int64_t next = row_at(off, n, 0, e);
+      if (next < ub + 32) break;
+      ub = next - 32;
+      continue;
+    }
+    const uint32_t base = gid && r < n ? uint32_t(vbase[gid[r]]) : 0u;
+    const int64_t stop = wend < e1 ? wend : e1;
+    const int len = int(stop - e);
+    const int rb = ob <= e ? 0 : (ob >= stop ? len : int(ob - e));
+    for (int x = lane; x - lane < len; x += 32 * SYM_BATCH) {
+      uint32_t t[SYM_BATCH];
+#pragma unroll
+      for (int j = 0; j < SYM_BATCH; ++j) t[j] = x + 32 * j < len ? __ldg(tgt + e + x + 32 * j) : 0u;
+#pragma unroll
+      for (int j = 0; j < SYM_BATCH; ++j) {
+        if (x - lane + 32 * j >= len) break;
+        const int at = x + 32 * j;
+        int pos = 0;
+#pragma unroll
+        for (int s = 16; s >= 1; s >>= 1)
+          if (__shfl_sync(FULL, rb, pos + s) <= at) pos += s;
+        const uint32_t u = uint32_t(ub + pos), v = t[j] + __shfl_sync(FULL, base, pos);
+        if (at < len && u != v) {
+          const unsigned long long h = mix64(uint64_t(u < v ? u : v) << 32 | (u < v ? v : u));
+          acc += u < v ? h : 0ull - h;
+        }
+      }
+    }
+    e = stop;
+  }
+  acc = warp_sum(acc);
+  if (lane == 0 && acc) atomicAdd(&rs->asym, acc);
 }
 
 __global__ void k_mod_square(const double *ctot, const uint32_t *labels, int64_t n, double *sums) {
@@ -698,14 +754,29 @@ cudaError_t launch_init_flags(uint8_t *aff0, uint8_t *aff1, const uint8_t *f, in
 
 // ctot: n doubles (zeroed by the caller), sums: 4 doubles (zeroed by the caller) receive
 // [internal weight, total weight 2M, sum of squared community totals, labels >= n seen].
+// Warps for m edges of n rows: at least 512 edges (or rows' worth) each, so that finding a warp's first row
+// stays a small part of its work.
+static int edge_blocks(int64_t n, int64_t m) {
+  const int64_t g = (m + MOD_ROW_COST * n + 512 * (TPB / 32) - 1) / (512 * (TPB / 32));
+  return int(g > 148 * 8 ? 148 * 8 : (g < 1 ? 1 : g));
+}
+
+cudaError_t launch_symmetry(const void *off, bool off64, const uint32_t *tgt, int64_t n, int64_t m, const uint32_t *gid,
+                            const int64_t *vbase, void *rs, cudaStream_t st) {
+  if (m <= 0) return cudaSuccess;
+  RunState *s = static_cast<RunState *>(rs);
+  const int g = edge_blocks(n, m);
+  if (off64) k_symmetry<int64_t><<<g, TPB, 0, st>>>(static_cast<const int64_t *>(off), tgt, n, m, gid, vbase, s);
+  else k_symmetry<int32_t><<<g, TPB, 0, st>>>(static_cast<const int32_t *>(off), tgt, n, m, gid, vbase, s);
+  return cudaGetLastError();
+}
+
 template <class O>
 static void launch_mod_edges(const O *off, const uint32_t *tgt, const float *wt, int64_t n, int64_t m,
                              const uint32_t *labels, double *ctot, double *sums, cudaStream_t st) {
-  // at least 512 edges a warp, so that finding a warp's first row stays a small part of its work
-  int64_t g = (m + MOD_ROW_COST * n + 512 * (TPB / 32) - 1) / (512 * (TPB / 32));
-  if (g > 148 * 8) g = 148 * 8;
-  if (wt) k_mod_edges<O, false><<<int(g), TPB, 0, st>>>(off, tgt, wt, n, m, labels, ctot, sums);
-  else k_mod_edges<O, true><<<int(g), TPB, 0, st>>>(off, tgt, wt, n, m, labels, ctot, sums);
+  const int g = edge_blocks(n, m);
+  if (wt) k_mod_edges<O, false><<<g, TPB, 0, st>>>(off, tgt, wt, n, m, labels, ctot, sums);
+  else k_mod_edges<O, true><<<g, TPB, 0, st>>>(off, tgt, wt, n, m, labels, ctot, sums);
 }
 
 cudaError_t launch_modularity(const void *off, bool off64, const uint32_t *tgt, const float *wt, int64_t n, int64_t m,

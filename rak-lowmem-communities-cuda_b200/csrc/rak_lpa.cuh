@@ -46,9 +46,14 @@ struct Counters {
 // vertex is processed, whatever its flag (the previous iteration marked no neighbours); nomark:
 // moved vertices mark no neighbours (the next iteration processes every vertex). Both false in
 // the other modes and in batches: the reference's pruning, flags marked by every move.
+// How a synchronous iteration's active set is found (LpaArgs::pull). pull_in: the flags read hold the
+// vertices that moved in the previous iteration, and a vertex is active if a neighbour's is set;
+// pull_out: this iteration's moves set the mover's own flag for that, and mark no neighbours.
 struct Phase {
   bool all;
   bool nomark;
+  bool pull_in;
+  bool pull_out;
 };
 
 template <class O>
@@ -673,20 +678,76 @@ __device__ __forceinline__ void choose(const LpaArgs &a, const Sketch<S> &sk, ui
   sk_choose<S, RULE>(sk, c, w);
 }
 
+// ---- the active set of a synchronous iteration, pulled ------------------------------------------
+//
+// On a symmetric graph a vertex has been marked exactly if one of its neighbours moved. Marking stores
+// a flag for every edge of every moved vertex -- and B200's L2 takes one store per 32-byte sector in
+// about 22 cycles, so the flags of a few popular vertices serialise: random flag stores measured 123
+// G/s over 2^20 flags, 44 over 2^16, 11 over 2^12, against 289 G/s for label gathers. When most vertices
+// move, looking for one neighbour that moved ends at the first or second edge instead. The kernel
+// chooses per iteration (lpa_run), on graphs whose symmetry the launch has checked (k_symmetry);
+// results are the same either way. Measured on B200 (synchronous split runs, marked -> pulled):
+// R-MAT scale 24 ef 16 77.6 -> 50.7 ms, scale 22 20.8 -> 12.5 ms, scale 20 ef 32 weighted 32.6 -> 13.8 ms, scale
+// 16 2.4 -> 1.6 ms, SBM 1 M vertices 4.1 -> 2.7 ms.
+
+// Whether a neighbour of u among edges [e, ee) moved; one lane, four edges in flight.
+__device__ __forceinline__ bool lane_pull(uint32_t u, int64_t e, int64_t ee, const uint32_t *tgt, const uint8_t *fin,
+                                          uint32_t base) {
+  constexpr int B = 4;
+  for (; e < ee; e += B) {
+    uint32_t t[B], any = 0;
+#pragma unroll
+    for (int j = 0; j < B; ++j) t[j] = e + j < ee ? base + ld_edge(tgt + e + j) : u;
+#pragma unroll
+    for (int j = 0; j < B; ++j) any |= t[j] != u ? uint32_t(fin[t[j]]) : 0u;
+    if (any) return true;
+  }
+  return false;
+}
+
+// The same by the aligned groups of G lanes, each for its own vertex (want: the group looks at all);
+// every lane of the warp calls it, and a group's lanes get the same answer.
+__device__ __forceinline__ bool group_pull(bool want, uint32_t u, int64_t eb, int64_t ee, int s, int G, int grp,
+                                           const uint32_t *tgt, const uint8_t *fin, uint32_t base) {
+  const unsigned gm = G == 32 ? FULL : ((1u << G) - 1u) << (grp * G);
+  bool found = false;
+  for (int64_t e = eb + s;; e += G) {
+    const bool more = want && !found && e < ee;
+    bool hit = false;
+    if (more) {
+      const uint32_t t = base + ld_edge(tgt + e);
+      hit = t != u && fin[t] != 0;
+    }
+    const unsigned hits = __ballot_sync(FULL, hit);
+    found = found || (hits & gm) != 0;
+    if (__ballot_sync(FULL, more && !found) == 0) return found;
+  }
+}
+
+// ---- work items: open (what to scan), close (choose, move) --------------------------------------
+
 // Region 6: one lane per vertex. Items are collected into a per-warp queue of active vertices
 // (inactive ones are settled at once), and the queue is processed 32 vertices at a time so every
 // lane has work; region 6 is sorted by degree, so a batch holds vertices of similar degree.
-template <int S, int MODE, class O, bool UNIT, bool BATCH>
-__device__ __forceinline__ int lane_collect(const LpaArgs &a, const Regions &rg, int64_t local, const uint32_t *vin,
-                                            uint32_t *vout, const uint8_t *fin, uint32_t *q, int qn, Phase ph) {
+template <class O, bool BATCH>
+__device__ __forceinline__ bool lane_active(const LpaArgs &a, const G_<O> &g, uint32_t u, const uint8_t *fin, Phase ph) {
+  uint32_t gi, base;
+  if (graph_of<BATCH>(a, u, gi, base)) return false;
+  if (ph.pull_in) return lane_pull(u, int64_t(__ldg(g.off + u)), int64_t(__ldg(g.off + u + 1)), g.tgt, fin, base);
+  return ph.all || fin[u] != 0;
+}
+
+template <int MODE, class O, bool BATCH>
+__device__ __forceinline__ int lane_collect(const LpaArgs &a, const Regions &rg, const G_<O> &g, int64_t local,
+                                            const uint32_t *vin, uint32_t *vout, const uint8_t *fin, uint32_t *q, int qn,
+                                            Phase ph) {
   const int lane = threadIdx.x & 31;
   const int64_t idx = local * 32 + lane;
   bool act = false;
   uint32_t u = 0;
   if (idx < rg.vcount[REG_LANE]) {
     u = __ldg(a.order + rg.vbegin[REG_LANE] + idx);
-    uint32_t gi, base;
-    act = (ph.all || fin[u] != 0) && !graph_of<BATCH>(a, u, gi, base);
+    act = lane_active<O, BATCH>(a, g, u, fin, ph);
     if constexpr (MODE != MODE_ASYNC)
       if (!act) vout[u] = vin[u];
   }
@@ -694,6 +755,32 @@ __device__ __forceinline__ int lane_collect(const LpaArgs &a, const Regions &rg,
   if (act) q[qn + __popc(m & ((1u << lane) - 1u))] = u;
   __syncwarp();
   return qn + __popc(m);
+}
+
+// The choice and move of an active vertex scanned by one lane; true if it moved.
+template <int S, int MODE, bool BATCH, int RULE>
+__device__ __forceinline__ bool lane_close(const LpaArgs &a, const Sketch<S> &sk, uint32_t u, uint32_t d, uint32_t gi,
+                                           uint32_t base, int64_t deg, int it, bool pickless, uint32_t *vout, uint8_t *fin,
+                                           uint8_t *fout, Counters &cnt, Phase ph) {
+  uint32_t c;
+  float w;
+  choose<S, RULE>(a, sk, u - base, it, c, w);
+  const bool moved = move_rule<S, RULE>(w, c, d, pickless);
+  cnt.processed += 1;
+  cnt.edges += (unsigned long long)deg;
+  if constexpr (MODE == MODE_ASYNC) {
+    fin[u] = 0;
+    if (moved) vout[u] = c;
+  } else {
+    vout[u] = moved ? c : d;
+    if (moved && ph.pull_out) fout[u] = 1;
+  }
+  if (moved) {
+    cnt.changed += 1;
+    cnt.moved_edges += (unsigned long long)deg;
+    count_move<BATCH>(a, gi, it);
+  }
+  return moved;
 }
 
 template <int S, int MODE, class O, bool UNIT, bool BATCH, int RULE>
@@ -714,75 +801,82 @@ __device__ __forceinline__ void lane_batch(const LpaArgs &a, const G_<O> &g, con
   else scan_range<S, UNIT, RULE, true>(sk, u, eb, ee, 1, g.tgt, g.wt, vin, base);
   if constexpr (MODE == MODE_SYNC && S > 1)
     if (a.rescan) rescan_range<S, UNIT>(sk, u, eb, ee, g.tgt, g.wt, vin, base);
-  uint32_t c;
-  float w;
-  choose<S, RULE>(a, sk, u - base, it, c, w);
-  const bool moved = move_rule<S, RULE>(w, c, d, pickless);
-  cnt.processed += 1;
-  cnt.edges += (unsigned long long)(ee - eb);
-  if constexpr (MODE == MODE_ASYNC) {
-    fin[u] = 0;
-    if (moved) vout[u] = c;
-  } else {
-    vout[u] = moved ? c : d;
-  }
-  if (moved) {
-    cnt.changed += 1;
-    cnt.moved_edges += (unsigned long long)(ee - eb);
-    count_move<BATCH>(a, gi, it);
-    if (ph.nomark) return;
-    if (!vec) mark_item<S>(a, u, eb, ee, 1, g.tgt, fout, base);
-    else if (mark_tested<S>(a)) mark_lane<true>(u, eb, ee, g.tgt, fout, base);
-    else mark_lane<false>(u, eb, ee, g.tgt, fout, base);
-  }
+  if (!lane_close<S, MODE, BATCH, RULE>(a, sk, u, d, gi, base, ee - eb, it, pickless, vout, fin, fout, cnt, ph)) return;
+  if (ph.nomark || ph.pull_out) return;
+  if (!vec) mark_item<S>(a, u, eb, ee, 1, g.tgt, fout, base);
+  else if (mark_tested<S>(a)) mark_lane<true>(u, eb, ee, g.tgt, fout, base);
+  else mark_lane<false>(u, eb, ee, g.tgt, fout, base);
 }
 
-// Regions 1..5: aligned groups of G lanes per vertex.
+// Regions 1..5: aligned groups of G lanes per vertex. A lane's view of its group's vertex.
+struct GroupVertex {
+  uint32_t u, d, gi, base;
+  int64_t eb, ee;
+  bool valid, active;
+};
+template <class O, bool BATCH>
+__device__ __forceinline__ GroupVertex group_open(const LpaArgs &a, const Regions &rg, const G_<O> &g, int r,
+                                                  int64_t local, const uint32_t *vin, const uint8_t *fin, Phase ph) {
+  const int G = region_group(r);
+  const int lane = threadIdx.x & 31, grp = lane / G, s = lane & (G - 1);
+  const int64_t idx = local * (32 / G) + grp;
+  GroupVertex v{0, 0, 0, 0, 0, 0, idx < rg.vcount[r], false};
+  if (v.valid) {
+    v.u = __ldg(a.order + rg.vbegin[r] + idx);
+    v.d = vin[v.u];
+    v.active = !graph_of<BATCH>(a, v.u, v.gi, v.base) && (ph.pull_in || ph.all || fin[v.u] != 0);
+    if (v.active) { v.eb = int64_t(__ldg(g.off + v.u)); v.ee = int64_t(__ldg(g.off + v.u + 1)); }
+  }
+  if (ph.pull_in) v.active = group_pull(v.active, v.u, v.eb, v.ee, s, G, grp, g.tgt, fin, v.base);
+  return v;
+}
+// Merges the group's sketches, chooses and moves; true on every lane of the group if it moved.
+template <int S, int MODE, bool BATCH, int RULE>
+__device__ __forceinline__ bool group_close(const LpaArgs &a, Sketch<S> &sk, const GroupVertex &v, int r, int it,
+                                            bool pickless, uint32_t *vout, uint8_t *fin, uint8_t *fout, Counters &cnt,
+                                            Phase ph) {
+  const int G = region_group(r);
+  const int lane = threadIdx.x & 31, grp = lane / G, s = lane & (G - 1);
+  if constexpr (MODE != MODE_SYNC) sk_tree<S, RULE>(sk, G);
+  uint32_t c;
+  float w;
+  choose<S, RULE>(a, sk, v.u - v.base, it, c, w);
+  bool moved = v.active && move_rule<S, RULE>(w, c, v.d, pickless);
+  moved = __shfl_sync(FULL, moved, grp * G);
+  if (s == 0 && v.valid) {
+    if (v.active) { cnt.processed += 1; cnt.edges += (unsigned long long)(v.ee - v.eb); }
+    if constexpr (MODE == MODE_ASYNC) {
+      if (v.active) fin[v.u] = 0;
+      if (moved) vout[v.u] = c;
+    } else {
+      vout[v.u] = moved ? c : v.d;
+      if (moved && ph.pull_out) fout[v.u] = 1;
+    }
+    if (moved) { cnt.changed += 1; cnt.moved_edges += (unsigned long long)(v.ee - v.eb); count_move<BATCH>(a, v.gi, it); }
+  }
+  return moved;
+}
+
 template <int S, int MODE, class O, bool UNIT, bool BATCH, int RULE>
 __device__ __forceinline__ void group_item(const LpaArgs &a, const Regions &rg, const G_<O> &g, int r, int64_t local,
                                            int it, bool pickless, const uint32_t *vin, uint32_t *vout,
                                            uint8_t *fin, uint8_t *fout, Counters &cnt, StageCtx &sc, Phase ph) {
   const int G = region_group(r);
   const int lane = threadIdx.x & 31, grp = lane / G, s = lane & (G - 1);
-  const int64_t idx = local * (32 / G) + grp;
-  const bool valid = idx < rg.vcount[r];
-  uint32_t u = 0, d = 0, gi = 0, base = 0;
-  int64_t eb = 0, ee = 0;
-  bool active = false;
-  if (valid) {
-    u = __ldg(a.order + rg.vbegin[r] + idx);
-    d = vin[u];
-    active = (ph.all || fin[u] != 0) && !graph_of<BATCH>(a, u, gi, base);
-    if (active) { eb = int64_t(__ldg(g.off + u)); ee = int64_t(__ldg(g.off + u + 1)); }
-  }
+  const GroupVertex v = group_open<O, BATCH>(a, rg, g, r, local, vin, fin, ph);
   Sketch<S> sk;
-  sk_clear<S, RULE>(sk, d);
+  sk_clear<S, RULE>(sk, v.d);
   if constexpr (MODE == MODE_SYNC) {
-    if (active) exact_group_scan<S, UNIT>(sk, u, eb, ee, G, grp, s, S > 1 && a.rescan, g.tgt, g.wt, vin, base);
+    if (v.active) exact_group_scan<S, UNIT>(sk, v.u, v.eb, v.ee, G, grp, s, S > 1 && a.rescan, g.tgt, g.wt, vin, v.base);
   } else {
     if (sc.on && G == 32)   // one vertex per warp: the warp's range is uniform
-      staged_scan<S, UNIT, RULE>(sk, sc, u, active ? eb : 0, active ? ee : 0, g.tgt, g.wt, vin, base,
+      staged_scan<S, UNIT, RULE>(sk, sc, v.u, v.active ? v.eb : 0, v.active ? v.ee : 0, g.tgt, g.wt, vin, v.base,
                                  static_cast<RunState *>(a.rs), a.timeout_ns);
-    else if (active)
-      scan_range<S, UNIT, RULE>(sk, u, eb + s, ee, G, g.tgt, g.wt, vin, base);
-    sk_tree<S, RULE>(sk, G);
+    else if (v.active)
+      scan_range<S, UNIT, RULE>(sk, v.u, v.eb + s, v.ee, G, g.tgt, g.wt, vin, v.base);
   }
-  uint32_t c;
-  float w;
-  choose<S, RULE>(a, sk, u - base, it, c, w);
-  bool moved = active && move_rule<S, RULE>(w, c, d, pickless);
-  moved = __shfl_sync(FULL, moved, grp * G);
-  if (s == 0 && valid) {
-    if (active) { cnt.processed += 1; cnt.edges += (unsigned long long)(ee - eb); }
-    if constexpr (MODE == MODE_ASYNC) {
-      if (active) fin[u] = 0;
-      if (moved) vout[u] = c;
-    } else {
-      vout[u] = moved ? c : d;
-    }
-    if (moved) { cnt.changed += 1; cnt.moved_edges += (unsigned long long)(ee - eb); count_move<BATCH>(a, gi, it); }
-  }
-  if (moved && !ph.nomark) mark_item<S>(a, u, eb + s, ee, G, g.tgt, fout, base);
+  const bool moved = group_close<S, MODE, BATCH, RULE>(a, sk, v, r, it, pickless, vout, fin, fout, cnt, ph);
+  if (moved && !ph.nomark && !ph.pull_out) mark_item<S>(a, v.u, v.eb + s, v.ee, G, g.tgt, fout, v.base);
 }
 
 // Region 0: one chunk of a split vertex per item. In the synchronous exact mode chunk 0's warp
@@ -790,127 +884,154 @@ __device__ __forceinline__ void group_item(const LpaArgs &a, const Regions &rg, 
 // warp builds a partial sketch (lane-strided, tree-merged), stores it, and the last chunk to
 // arrive merges all partial sketches in a fixed order and makes the move; its neighbours are
 // marked in a second phase after the iteration's barrier.
+struct HubChunk {
+  uint32_t h, u, gi, base;
+  int64_t first, nch, j;   // the vertex's first chunk and chunks, this one's index among them
+  int64_t eb, ee, cb, ce;  // edges of the vertex and of the chunk
+  bool active;
+};
+template <int MODE, class O, bool BATCH>
+__device__ __forceinline__ HubChunk hub_open(const LpaArgs &a, const Regions &rg, const G_<O> &g, int64_t local, int it,
+                                             uint8_t *fin, Phase ph) {
+  const int lane = threadIdx.x & 31;
+  HubChunk k;
+  k.h = __ldg(a.chunk_hub + local);
+  k.first = __ldg(a.hub_first + k.h);
+  k.nch = __ldg(a.hub_first + k.h + 1) - k.first;
+  k.j = local - k.first;
+  k.u = __ldg(a.order + rg.vbegin[REG_HUB] + k.h);
+  k.eb = int64_t(__ldg(g.off + k.u));
+  k.ee = int64_t(__ldg(g.off + k.u + 1));
+  k.cb = k.eb + k.j * a.hub_chunk;
+  k.ce = k.cb + a.hub_chunk < k.ee ? k.cb + a.hub_chunk : k.ee;
+  const bool gfin = graph_of<BATCH>(a, k.u, k.gi, k.base);  // stable within an iteration
+  if (gfin) {
+    k.active = false;
+  } else if (MODE != MODE_ASYNC) {
+    k.active = ph.pull_in ? group_pull(true, k.u, k.eb, k.ee, lane, 32, 0, g.tgt, fin, k.base) : fin[k.u] != 0;
+  } else {
+    // All chunks of u agree on whether u is processed this iteration: the first chunk to get
+    // here decides from u's flag (and clears it); the others read the decision.
+    unsigned int dec = 0;
+    if (lane == 0) {
+      const unsigned int tag = unsigned(it + 1);
+      unsigned int cur = *(volatile unsigned int *)(a.hub_claim + k.h);
+      if ((cur >> 1) != tag) {
+        const unsigned int want = (tag << 1) | (ph.all || *(volatile uint8_t *)(fin + k.u) ? 1u : 0u);
+        const unsigned int prev = atomicCAS(a.hub_claim + k.h, cur, want);
+        if (prev == cur) {
+          cur = want;
+          if (want & 1u) fin[k.u] = 0;
+        } else {
+          cur = prev;
+        }
+      }
+      dec = cur & 1u;
+    }
+    k.active = __shfl_sync(FULL, dec, 0) != 0;
+  }
+  return k;
+}
+// sk: the warp's lanes' sketches of the chunk (d0: what a clear sketch starts from).
+template <int S, int MODE, bool BATCH, int RULE>
+__device__ __forceinline__ void hub_close(const LpaArgs &a, Sketch<S> &sk, const HubChunk &k, uint32_t d0, int64_t local,
+                                          int it, bool pickless, const uint32_t *vin, uint32_t *vout, uint8_t *fout,
+                                          Counters &cnt, Phase ph) {
+  const int lane = threadIdx.x & 31;
+  sk_tree<S, RULE>(sk, 32);
+  unsigned int last = 0;
+  if (lane == 0) {
+    if (k.active) {
+      cnt.edges += (unsigned long long)(k.ce - k.cb);
+#pragma unroll
+      for (int i = 0; i < S; ++i) {
+        a.sk_keys[local * S + i] = sk.k[i];
+        a.sk_wts[local * S + i] = sk.w[i];
+      }
+    }
+    __threadfence();
+    last = atomicAdd(a.hub_arrive + k.h, 1u) == unsigned(k.nch - 1);
+  }
+  last = __shfl_sync(FULL, last, 0);
+  if (!last) return;
+  __threadfence();
+  if (lane == 0) a.hub_arrive[k.h] = 0;
+  const uint32_t d = vin[k.u];
+  if (!k.active) {
+    if (MODE != MODE_ASYNC && lane == 0) vout[k.u] = d;
+    return;
+  }
+  Sketch<S> acc;
+  sk_clear<S, RULE>(acc, d0);
+  for (int64_t jj = lane; jj < k.nch; jj += 32) {
+    uint32_t bk[S];
+    float bw[S];
+#pragma unroll
+    for (int i = 0; i < S; ++i) {
+      bk[i] = __ldcg(a.sk_keys + (k.first + jj) * S + i);
+      bw[i] = __ldcg(a.sk_wts + (k.first + jj) * S + i);
+    }
+    sk_merge<S, RULE>(acc, bk, bw);
+  }
+  sk_tree<S, RULE>(acc, 32);
+  if (lane == 0) {
+    uint32_t c;
+    float w;
+    choose<S, RULE>(a, acc, k.u - k.base, it, c, w);
+    const bool moved = move_rule<S, RULE>(w, c, d, pickless);
+    cnt.processed += 1;
+    if constexpr (MODE == MODE_ASYNC) {
+      if (moved) vout[k.u] = c;
+    } else {
+      vout[k.u] = moved ? c : d;
+      if (moved && ph.pull_out) fout[k.u] = 1;
+    }
+    if (moved) {
+      cnt.changed += 1;
+      cnt.moved_edges += (unsigned long long)(k.ee - k.eb);
+      count_move<BATCH>(a, k.gi, it);
+      a.hub_moved[k.h] = it;
+      atomicAdd(a.stats + STATS_STRIDE * it + STAT_HUBS_MOVED, 1ull);
+    }
+  }
+}
+
 template <int S, int MODE, class O, bool UNIT, bool BATCH, int RULE>
 __device__ __forceinline__ void hub_item(const LpaArgs &a, const Regions &rg, const G_<O> &g, int64_t local, int it, bool pickless,
                                          const uint32_t *vin, uint32_t *vout, uint8_t *fin, uint8_t *fout,
                                          Counters &cnt, StageCtx &sc, Phase ph) {
   const int lane = threadIdx.x & 31;
-  const uint32_t h = __ldg(a.chunk_hub + local);
-  const int64_t first = __ldg(a.hub_first + h), nch = __ldg(a.hub_first + h + 1) - first, j = local - first;
-  const uint32_t u = __ldg(a.order + rg.vbegin[REG_HUB] + h);
-  const int64_t eb = int64_t(__ldg(g.off + u)), ee = int64_t(__ldg(g.off + u + 1));
-  uint32_t gi, base;
-  const bool gfin = graph_of<BATCH>(a, u, gi, base);  // stable within an iteration
   if constexpr (MODE == MODE_SYNC) {
-    if (j != 0) return;
-    const uint32_t d = vin[u];
-    const bool active = fin[u] != 0 && !gfin;
+    if (local != __ldg(a.hub_first + __ldg(a.chunk_hub + local))) return;
+    const HubChunk k = hub_open<MODE, O, BATCH>(a, rg, g, local, it, fin, ph);
+    const uint32_t d = vin[k.u];
     Sketch<S> sk;
     sk_clear<S, RULE>(sk, d);
-    if (active) exact_group_scan<S, UNIT>(sk, u, eb, ee, 32, 0, lane, S > 1 && a.rescan, g.tgt, g.wt, vin, base);
+    if (k.active) exact_group_scan<S, UNIT>(sk, k.u, k.eb, k.ee, 32, 0, lane, S > 1 && a.rescan, g.tgt, g.wt, vin, k.base);
     uint32_t c;
     float w;
-    choose<S, RULE>(a, sk, u - base, it, c, w);
-    const bool moved = active && move_rule<S, RULE>(w, c, d, pickless);
+    choose<S, RULE>(a, sk, k.u - k.base, it, c, w);
+    const bool moved = k.active && move_rule<S, RULE>(w, c, d, pickless);
     if (lane == 0) {
-      vout[u] = moved ? c : d;
-      if (active) { cnt.processed += 1; cnt.edges += (unsigned long long)(ee - eb); }
-      if (moved) { cnt.changed += 1; cnt.moved_edges += (unsigned long long)(ee - eb); count_move<BATCH>(a, gi, it); }
+      vout[k.u] = moved ? c : d;
+      if (moved && ph.pull_out) fout[k.u] = 1;
+      if (k.active) { cnt.processed += 1; cnt.edges += (unsigned long long)(k.ee - k.eb); }
+      if (moved) { cnt.changed += 1; cnt.moved_edges += (unsigned long long)(k.ee - k.eb); count_move<BATCH>(a, k.gi, it); }
     }
-    if (moved) mark_item<S>(a, u, eb + lane, ee, 32, g.tgt, fout, base);
+    if (moved && !ph.pull_out) mark_item<S>(a, k.u, k.eb + lane, k.ee, 32, g.tgt, fout, k.base);
     return;
   } else {
-    bool active;
-    if (gfin) {
-      active = false;
-    } else if constexpr (MODE == MODE_SPLIT) {
-      active = fin[u] != 0;
-    } else {
-      // All chunks of u agree on whether u is processed this iteration: the first chunk to get
-      // here decides from u's flag (and clears it); the others read the decision.
-      unsigned int dec = 0;
-      if (lane == 0) {
-        const unsigned int tag = unsigned(it + 1);
-        unsigned int cur = *(volatile unsigned int *)(a.hub_claim + h);
-        if ((cur >> 1) != tag) {
-          const unsigned int want = (tag << 1) | (ph.all || *(volatile uint8_t *)(fin + u) ? 1u : 0u);
-          const unsigned int prev = atomicCAS(a.hub_claim + h, cur, want);
-          if (prev == cur) {
-            cur = want;
-            if (want & 1u) fin[u] = 0;
-          } else {
-            cur = prev;
-          }
-        }
-        dec = cur & 1u;
-      }
-      active = __shfl_sync(FULL, dec, 0) != 0;
-    }
+    const HubChunk k = hub_open<MODE, O, BATCH>(a, rg, g, local, it, fin, ph);
     // Boyer-Moore under the GPU rules starts every partial vote from u's label
-    const uint32_t d0 = (S == 1 && RULE == RULE_GPU) ? vin[u] : NONE;
+    const uint32_t d0 = (S == 1 && RULE == RULE_GPU) ? vin[k.u] : NONE;
     Sketch<S> sk;
     sk_clear<S, RULE>(sk, d0);
-    const int64_t cb = eb + j * a.hub_chunk, ce = cb + a.hub_chunk < ee ? cb + a.hub_chunk : ee;
     if (sc.on)   // active is the same on every lane
-      staged_scan<S, UNIT, RULE>(sk, sc, u, active ? cb : 0, active ? ce : 0, g.tgt, g.wt, vin, base,
+      staged_scan<S, UNIT, RULE>(sk, sc, k.u, k.active ? k.cb : 0, k.active ? k.ce : 0, g.tgt, g.wt, vin, k.base,
                                  static_cast<RunState *>(a.rs), a.timeout_ns);
-    else if (active)
-      scan_range<S, UNIT, RULE>(sk, u, cb + lane, ce, 32, g.tgt, g.wt, vin, base);
-    sk_tree<S, RULE>(sk, 32);
-    unsigned int last = 0;
-    if (lane == 0) {
-      if (active) {
-        cnt.edges += (unsigned long long)(ce - cb);
-#pragma unroll
-        for (int i = 0; i < S; ++i) {
-          a.sk_keys[local * S + i] = sk.k[i];
-          a.sk_wts[local * S + i] = sk.w[i];
-        }
-      }
-      __threadfence();
-      last = atomicAdd(a.hub_arrive + h, 1u) == unsigned(nch - 1);
-    }
-    last = __shfl_sync(FULL, last, 0);
-    if (!last) return;
-    __threadfence();
-    if (lane == 0) a.hub_arrive[h] = 0;
-    const uint32_t d = vin[u];
-    if (!active) {
-      if (MODE != MODE_ASYNC && lane == 0) vout[u] = d;
-      return;
-    }
-    Sketch<S> acc;
-    sk_clear<S, RULE>(acc, d0);
-    for (int64_t jj = lane; jj < nch; jj += 32) {
-      uint32_t bk[S];
-      float bw[S];
-#pragma unroll
-      for (int i = 0; i < S; ++i) {
-        bk[i] = __ldcg(a.sk_keys + (first + jj) * S + i);
-        bw[i] = __ldcg(a.sk_wts + (first + jj) * S + i);
-      }
-      sk_merge<S, RULE>(acc, bk, bw);
-    }
-    sk_tree<S, RULE>(acc, 32);
-    if (lane == 0) {
-      uint32_t c;
-      float w;
-      choose<S, RULE>(a, acc, u - base, it, c, w);
-      const bool moved = move_rule<S, RULE>(w, c, d, pickless);
-      cnt.processed += 1;
-      if constexpr (MODE == MODE_ASYNC) {
-        if (moved) vout[u] = c;
-      } else {
-        vout[u] = moved ? c : d;
-      }
-      if (moved) {
-        cnt.changed += 1;
-        cnt.moved_edges += (unsigned long long)(ee - eb);
-        count_move<BATCH>(a, gi, it);
-        a.hub_moved[h] = it;
-        atomicAdd(a.stats + STATS_STRIDE * it + STAT_HUBS_MOVED, 1ull);
-      }
-    }
+    else if (k.active)
+      scan_range<S, UNIT, RULE>(sk, k.u, k.cb + lane, k.ce, 32, g.tgt, g.wt, vin, k.base);
+    hub_close<S, MODE, BATCH, RULE>(a, sk, k, d0, local, it, pickless, vin, vout, fout, cnt, ph);
   }
 }
 
@@ -967,7 +1088,8 @@ __global__ void __launch_bounds__(256, RAK_MIN_BLOCKS) lpa_run(const LpaArgs a) 
   // frontier would hold nearly every vertex anyway, and the marking it saves is a re-read of each
   // moved vertex's edges plus a random flag access per edge. Decided from the previous iteration's
   // counter, which every block reads after the barrier, so all blocks agree.
-  Phase ph{false, false};
+  Phase ph{false, false, false, false};
+  const bool can_pull = MODE != MODE_ASYNC && a.pull != 0 && __ldcg(&rs->asym) == 0ull;
   for (int it = 0; it < a.iters; ++it) {
     if (threadIdx.x < 4) blk[threadIdx.x] = 0;
     if constexpr (MODE == MODE_ASYNC && !BATCH) {
@@ -976,6 +1098,15 @@ __global__ void __launch_bounds__(256, RAK_MIN_BLOCKS) lpa_run(const LpaArgs a) 
                   __ldcg(a.stats + STATS_STRIDE * (it - 1) + STAT_MOVED_EDGES) >= a.dense_moved_edges;
       if (blockIdx.x == 0 && threadIdx.x == 0)
         a.stats[STATS_STRIDE * it + STAT_PHASE] = (ph.all ? 2ull : 0ull) | (ph.nomark ? 1ull : 0ull);
+    }
+    if constexpr (MODE != MODE_ASYNC) {
+      // Pull when the previous iteration's moved vertices hold a quarter of the edges or more (in the
+      // first iteration: when every vertex starts affected). Every block reads the same counter after
+      // the barrier, so all blocks agree; the choice changes what the next iteration reads, not its result.
+      ph.pull_in = ph.pull_out;
+      ph.pull_out = can_pull && it + 1 < a.iters &&
+                    (it == 0 ? a.all_flags != 0
+                             : __ldcg(a.stats + STATS_STRIDE * (it - 1) + STAT_MOVED_EDGES) * 4ull >= (unsigned long long)a.m);
     }
     __syncthreads();
     const int l = a.start_iter + it;
@@ -1002,7 +1133,7 @@ __global__ void __launch_bounds__(256, RAK_MIN_BLOCKS) lpa_run(const LpaArgs a) 
         for (int64_t sb = 0; sb < rg.lane_item; ++sb) {
           const int64_t sub = local * rg.lane_item + sb;
           if (sub * 32 >= rg.vcount[REG_LANE]) break;
-          qn = lane_collect<S, MODE, O, UNIT, BATCH>(a, rg, sub, vin, vout, fin, q, qn, ph);
+          qn = lane_collect<MODE, O, BATCH>(a, rg, g, sub, vin, vout, fin, q, qn, ph);
           if (qn >= 32) {
             RAK_BY_RULE(lane_batch, (a, g, q, 32, it, pickless, vin, vout, fin, fout, cnt, ph));
             __syncwarp();
@@ -1041,7 +1172,7 @@ __global__ void __launch_bounds__(256, RAK_MIN_BLOCKS) lpa_run(const LpaArgs a) 
     const bool done = !BATCH && (it + 1 >= a.iters || (test && double(changed) / double(a.n) <= a.tolerance));
     // The synchronous split mode completes the next flags even on the last iteration, so a
     // single step returns them whole.
-    if (MODE != MODE_SYNC && !ph.nomark && (!done || MODE == MODE_SPLIT) && a.nchunks > 0 &&
+    if (MODE != MODE_SYNC && !ph.nomark && !ph.pull_out && (!done || MODE == MODE_SPLIT) && a.nchunks > 0 &&
         __ldcg(a.stats + STATS_STRIDE * it + STAT_HUBS_MOVED) > 0) {
       // Second phase: neighbours of split vertices that moved this iteration.
       for (int64_t i = gw; i < a.nchunks; i += nw) {

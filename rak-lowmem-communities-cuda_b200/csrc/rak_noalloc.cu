@@ -276,7 +276,7 @@ extern "C" rak_status rak_lowmem_cuda_noalloc(int device, void *stream, const ra
   else NA_TRY(launch_init(membership, vcom1, q, n, st));
   NA_TRY(launch_init_flags(aff0, aff1, o->initial_flags, n, st));
   LpaArgs a{};
-  a.off = g->offsets; a.tgt = g->targets; a.wt = g->weights; a.n = n;
+  a.off = g->offsets; a.tgt = g->targets; a.wt = g->weights; a.n = n; a.m = g->m;
   a.order = order; a.rg = rg;
   a.chunk_hub = chunk_hub; a.hub_first = first; a.hub_chunk = ly.hub_chunk; a.nchunks = nchunks;
   a.vcom0 = membership; a.vcom1 = vcom1; a.aff0 = aff0; a.aff1 = aff1;
@@ -296,6 +296,8 @@ extern "C" rak_status rak_lowmem_cuda_noalloc(int device, void *stream, const ra
   a.grid_cap = o->max_blocks > 0 ? o->max_blocks : 0;
   a.timeout_ns = o->wait_timeout_ns > 0 ? (long long)o->wait_timeout_ns : DEFAULT_WAIT_TIMEOUT_NS;
   a.dense_moved_edges = dense_threshold(mode, o->dense_pct, g->m);
+  a.pull = pull_for(mode, iters, g->m); a.all_flags = o->initial_flags == nullptr;
+  if (a.pull) NA_TRY(launch_symmetry(g->offsets, off64, g->targets, n, g->m, nullptr, nullptr, rs, st));
   if (iters > 0) {
     int grid = 0;
     NA_TRY(launch_lpa(a, slots, mode, off64, st, &grid));
