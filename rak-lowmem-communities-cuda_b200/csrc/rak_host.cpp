@@ -381,7 +381,7 @@ rak_status validate_host_t(const O *off, const uint32_t *tgt, int64_t n, int64_t
 int nkeys_of(const Layout &ly) { return int(6 + ly.lane_max + 1); }
 
 // Region sizes, item counts and chunk table from the key histogram and split-vertex degrees.
-void regions_from(const std::vector<unsigned long long> &hist, const Layout &ly, int64_t nchunks, int sms,
+void regions_from(const std::vector<unsigned long long> &hist, const Layout &ly, int64_t m, int64_t nchunks, int sms,
                   rak::Regions *rg) {
   int64_t cnt[rak::NREG] = {};
   for (int k = 0; k < 6; ++k) cnt[k] = int64_t(hist[k]);
@@ -396,6 +396,7 @@ void regions_from(const std::vector<unsigned long long> &hist, const Layout &ly,
     it += rak::region_items(r, cnt[r], nchunks, rg->lane_item);
   }
   rg->ibegin[rak::NREG] = it;
+  rak::set_wide(rg, hist.data(), ly, m);
 }
 
 rak_status build_plan(rak_ctx *ctx, rak_graph *gr, const Layout &ly, Tracker *tr) {
@@ -455,7 +456,7 @@ rak_status build_plan(rak_ctx *ctx, rak_graph *gr, const Layout &ly, Tracker *tr
     RAK_TRY(ctx, cudaMemcpyAsync(gr->chunk_hub, ch.data(), ch.size() * 4, cudaMemcpyHostToDevice, st));
   }
   gr->plan_bytes = gr->p_order.bytes + gr->p_hub_first.bytes + gr->p_chunk_hub.bytes;
-  regions_from(h, ly, gr->nchunks, ctx->sms, &gr->rg);
+  regions_from(h, ly, gr->m, gr->nchunks, ctx->sms, &gr->rg);
   cudaEventRecord(ev.e[1], st);
   RAK_TRY(ctx, cudaStreamSynchronize(st));
   gr->plan_ms = ev.ms(0, 1);
@@ -585,7 +586,7 @@ rak_status run_resident(rak_ctx *ctx, rak_graph *gr, const uint32_t *q, const ui
   RAK_TRY(ctx, ensure(b.skk, nc * size_t(r.slots) * 4));
   RAK_TRY(ctx, ensure(b.skw, nc * size_t(r.slots) * 4));
   RAK_TRY(ctx, ensure(b.stats, size_t(iters) * rak::STATS_STRIDE * 8));
-  RAK_TRY(ctx, ensure(b.rs, sizeof(rak::RunStateHost)));
+  RAK_TRY(ctx, ensure(b.rs, rak::RUN_STATE_BYTES));
   // asynchronous id-label runs work on the graph renumbered in work order (rak_renumber.cu)
   // by default only resident graphs, run again and again, pay for the copy (R-MAT scale 27: about
   // 80 ms once, 26 ms less per run), and only large dense ones: on a sparse R-MAT (scale 25, average
@@ -617,7 +618,7 @@ rak_status run_resident(rak_ctx *ctx, rak_graph *gr, const uint32_t *q, const ui
   a.sk_keys = b.skk.as<uint32_t>(); a.sk_wts = b.skw.as<float>();
   a.stats = b.stats.as<unsigned long long>(); a.rs = b.rs.p;
   a.iters = r.iters; a.start_iter = r.start; a.tolerance = r.tol; a.pickless_step = r.pickless;
-  a.check_on_pickless = r.check_on_pickless; a.rescan = r.rescan; a.mark_test = rak::mark_test_for(a.n, gr->m); a.gpu_rule = r.rule == 2; a.timeout_ns = r.timeout_ns; a.tie_until = r.tie_until; a.stage = r.stage; a.grid_cap = r.max_blocks;
+  a.check_on_pickless = r.check_on_pickless; a.rescan = r.rescan; a.mark_test = rak::mark_test_for(a.n, gr->m); a.gpu_rule = r.rule == 2; a.alt = rak::alt_for(r.slots, r.mode, a.gpu_rule, false, n, gr->m, gr->ly, gr->rg); a.timeout_ns = r.timeout_ns; a.tie_until = r.tie_until; a.stage = r.stage; a.grid_cap = r.max_blocks;
   a.dense_moved_edges = rak::dense_threshold(r.mode, r.dense_pct, gr->m);
   a.pull = rak::pull_for(r.mode, r.iters, gr->m); a.all_flags = flags == nullptr;
   if (renum) {
@@ -627,7 +628,7 @@ rak_status run_resident(rak_ctx *ctx, rak_graph *gr, const uint32_t *q, const ui
   }
 
   // the kernel's module is loaded here, not inside the timed region
-  if (r.iters > 0) RAK_TRY(ctx, rak::prepare_lpa(r.slots, r.mode, gr->off64, gr->wt == nullptr, false, r.stage));
+  if (r.iters > 0) RAK_TRY(ctx, rak::prepare_lpa(r.slots, r.mode, gr->off64, gr->wt == nullptr, false, r.stage, a.alt));
   // Labels as positions in the reference GPU path's vertex order (inc/rakLowmemCuda.hxx:563,
   // 591-592), so that its pickless rule compares the same label order; turned back into vertex ids
   // after the run. The order depends on degrees only: built once per graph.
@@ -950,7 +951,7 @@ rak_status rak_graph_step(rak_ctx *ctx, rak_graph *gr, const rak_options *o, int
   RAK_TRY(ctx, b.skk.alloc(nc * size_t(r.slots) * 4, nullptr));
   RAK_TRY(ctx, b.skw.alloc(nc * size_t(r.slots) * 4, nullptr));
   RAK_TRY(ctx, b.stats.alloc(rak::STATS_STRIDE * 8, nullptr));
-  RAK_TRY(ctx, b.rs.alloc(sizeof(rak::RunStateHost), nullptr));
+  RAK_TRY(ctx, b.rs.alloc(rak::RUN_STATE_BYTES, nullptr));
   RAK_TRY(ctx, cudaMemsetAsync(b.arrive.p, 0, b.arrive.bytes, st));
   RAK_TRY(ctx, cudaMemsetAsync(b.claim.p, 0, b.claim.bytes, st));
   RAK_TRY(ctx, cudaMemsetAsync(b.moved.p, 0xFF, b.moved.bytes, st));
@@ -973,7 +974,7 @@ rak_status rak_graph_step(rak_ctx *ctx, rak_graph *gr, const rak_options *o, int
   a.sk_keys = b.skk.as<uint32_t>(); a.sk_wts = b.skw.as<float>();
   a.stats = b.stats.as<unsigned long long>(); a.rs = b.rs.p;
   a.iters = 1; a.start_iter = iteration; a.tolerance = r.tol; a.pickless_step = r.pickless;
-  a.check_on_pickless = r.check_on_pickless; a.rescan = r.rescan; a.mark_test = rak::mark_test_for(a.n, gr->m); a.gpu_rule = r.rule == 2; a.timeout_ns = r.timeout_ns; a.tie_until = r.tie_until; a.stage = r.stage; a.grid_cap = r.max_blocks;
+  a.check_on_pickless = r.check_on_pickless; a.rescan = r.rescan; a.mark_test = rak::mark_test_for(a.n, gr->m); a.gpu_rule = r.rule == 2; a.alt = rak::alt_for(r.slots, r.mode, a.gpu_rule, false, n, gr->m, gr->ly, gr->rg); a.timeout_ns = r.timeout_ns; a.tie_until = r.tie_until; a.stage = r.stage; a.grid_cap = r.max_blocks;
   int grid = 0;
   RAK_TRY(ctx, rak::launch_lpa(a, r.slots, r.mode, gr->off64, st, &grid));
   unsigned long long s[rak::STATS_STRIDE] = {};
@@ -1202,7 +1203,8 @@ namespace {
 rak_status batch_prepare(rak_ctx *ctx, rak_batch *b, const Resolved &r) {
   rak_graph *gr = b->g;
   if (!same_layout(gr->ly, r.ly)) RAK_CHECK(build_plan(ctx, gr, r.ly, nullptr));
-  if (r.iters > 0) RAK_TRY(ctx, rak::prepare_lpa(r.slots, r.mode, true, gr->wt == nullptr, true, r.stage));
+  if (r.iters > 0) RAK_TRY(ctx, rak::prepare_lpa(r.slots, r.mode, true, gr->wt == nullptr, true, r.stage,
+                                                rak::alt_for(r.slots, r.mode, r.rule == 2, true, gr->n, gr->m, gr->ly, gr->rg)));
   const int64_t n = gr->n, G = b->ngraphs;
   const bool sync = r.mode != RAK_MODE_ASYNC;
   const int iters = std::max(r.iters, 1);
@@ -1219,7 +1221,7 @@ rak_status batch_prepare(rak_ctx *ctx, rak_batch *b, const Resolved &r) {
   RAK_TRY(ctx, ensure(rb.skk, nc * size_t(r.slots) * 4));
   RAK_TRY(ctx, ensure(rb.skw, nc * size_t(r.slots) * 4));
   RAK_TRY(ctx, ensure(rb.stats, size_t(iters) * rak::STATS_STRIDE * 8));
-  RAK_TRY(ctx, ensure(rb.rs, sizeof(rak::RunStateHost)));
+  RAK_TRY(ctx, ensure(rb.rs, rak::RUN_STATE_BYTES));
   RAK_TRY(ctx, ensure(b->vcom0, size_t(n) * 4 + 16));
   RAK_TRY(ctx, ensure(b->gdone, size_t(G) + 16));
   RAK_TRY(ctx, ensure(b->giters, size_t(G) * 4 + 16));
@@ -1256,7 +1258,7 @@ rak_status batch_enqueue(rak_ctx *ctx, rak_batch *b, const uint32_t *q, const Re
   RAK_TRY(ctx, cudaMemsetAsync(rb.claim.p, 0, rb.claim.bytes, st));
   RAK_TRY(ctx, cudaMemsetAsync(rb.moved.p, 0xFF, rb.moved.bytes, st));
   RAK_TRY(ctx, cudaMemsetAsync(rb.stats.p, 0, size_t(iters) * rak::STATS_STRIDE * 8, st));
-  RAK_TRY(ctx, cudaMemsetAsync(rb.rs.p, 0, sizeof(rak::RunStateHost), st));
+  RAK_TRY(ctx, cudaMemsetAsync(rb.rs.p, 0, rak::RUN_STATE_BYTES, st));
   RAK_TRY(ctx, cudaMemsetAsync(b->gdone.p, 0, size_t(G) + 16, st));
   RAK_TRY(ctx, cudaMemsetAsync(b->giters.p, 0, size_t(G) * 4 + 16, st));
   RAK_TRY(ctx, cudaMemsetAsync(b->gchanged.p, 0, size_t(G) * 16 + 16, st));
@@ -1282,7 +1284,7 @@ rak_status batch_enqueue(rak_ctx *ctx, rak_batch *b, const uint32_t *q, const Re
     a.giters = b->giters.as<int32_t>(); a.gchanged = b->gchanged.as<unsigned long long>();
     a.running = b->running.as<unsigned int>(); a.ngraphs = G; a.grid_cap = grid_cap > 0 ? grid_cap : r.max_blocks;
     a.iters = r.iters; a.start_iter = r.start; a.tolerance = r.tol; a.pickless_step = r.pickless;
-    a.check_on_pickless = r.check_on_pickless; a.rescan = r.rescan; a.mark_test = rak::mark_test_for_batch(a.n, gr->m, G); a.gpu_rule = r.rule == 2; a.timeout_ns = r.timeout_ns; a.tie_until = r.tie_until; a.stage = r.stage;
+    a.check_on_pickless = r.check_on_pickless; a.rescan = r.rescan; a.mark_test = rak::mark_test_for_batch(a.n, gr->m, G); a.gpu_rule = r.rule == 2; a.alt = rak::alt_for(r.slots, r.mode, a.gpu_rule, true, n, gr->m, gr->ly, gr->rg); a.timeout_ns = r.timeout_ns; a.tie_until = r.tie_until; a.stage = r.stage;
     a.pull = rak::pull_for(r.mode, r.iters, gr->m); a.all_flags = 1;
     if (a.pull) RAK_TRY(ctx, rak::launch_symmetry(gr->off, true, gr->tgt, n, gr->m, a.gid, a.vbase, rb.rs.p, st));
     int grid = 0;

@@ -3,6 +3,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <cstddef>
 #include <cstdint>
 
 namespace rak {
@@ -42,6 +43,10 @@ struct Regions {
   int64_t vcount[NREG];
   int64_t ibegin[NREG + 1];  // item prefix; ibegin[NREG] = total items
   int64_t lane_item;         // batches of 32 one-lane vertices per item (lane_item_for)
+  // wide items (rak_lpa.cuh), the first ones: every item before region 6 and the first wide_lanes batches
+  // of region 6 (wide_all), or those items of regions 0 and 1 whose chains exceed wide_len
+  int64_t wide_items, wide_lanes;
+  int wide_len, wide_all;
 };
 
 // Layout parameters (rak_options lane_max / hub_min / hub_chunk after defaults).
@@ -66,6 +71,40 @@ constexpr int DEFAULT_DENSE_PCT = -1;
 // Bound on each device-side wait when rak_options.wait_timeout_ns is 0.
 constexpr long long DEFAULT_WAIT_TIMEOUT_NS = 20LL * 1000 * 1000 * 1000;
 
+// Chains -- the edges one sketch takes -- longer than m >> 16 (never 8 or fewer) are scanned by a block instead
+// of a warp (rak_lpa.cuh). A block's scan costs more instructions, a warp's takes longer, and a balanced
+// iteration of m edges lasts about m / 250 G/s. Below lane_max that means every item before region 6 and region
+// 6's vertices of higher degree; above it the chains of regions 0 and 1, the only longer ones. Measured on B200
+// with the line at m >> 18 / 16 / 14: R-MAT scale 16 1.24 / 1.04 / 0.96 ms, scale 18 2.33 / 2.19 / 2.66 ms, scale
+// 20 7.1 / 6.5 / 6.9 ms, scale 20 ef 32 weighted 14.1 / 9.8 / 13.9 ms, scale 22 13.3 / 12.5 / 12.5 ms.
+constexpr int WIDE_MIN = 8;
+// hist: vertices per plan key (plan_key); rg: its other fields set.
+inline void set_wide(Regions *rg, const unsigned long long *hist, const Layout &ly, int64_t m) {
+  const int64_t len = (m >> 16) > WIDE_MIN ? m >> 16 : WIDE_MIN;
+  rg->wide_len = int(len < (int64_t(1) << 26) ? len : (int64_t(1) << 26));
+  rg->wide_all = len < ly.lane_max;
+  rg->wide_lanes = 0;
+  if (rg->wide_all) {
+    int64_t v = 0;
+    for (int64_t deg = len + 1; deg <= ly.lane_max; ++deg) v += int64_t(hist[6 + ly.lane_max - deg]);
+    rg->wide_lanes = v / 32 / rg->lane_item * rg->lane_item;
+    rg->wide_items = rg->ibegin[REG_LANE] + rg->wide_lanes;
+  } else {
+    const int64_t most = ly.hub_min > ly.hub_chunk ? ly.hub_min : ly.hub_chunk;
+    rg->wide_items = most > 32 * int64_t(rg->wide_len) ? rg->ibegin[2] : 0;
+  }
+}
+// Whether a launch takes the other kernel of its mode (resolve_lpa_slots). Synchronous split runs: the one that
+// scans wide items -- there are some, Misra-Gries under the CPU rules, chains short enough for whole-number unit
+// weights (2^24 edges). Asynchronous runs: the faster lpa_run, for Misra-Gries on one graph of those that
+// mark_test_for names (rak_lpa_async.cuh says why not for the others).
+inline int mark_test_for(int64_t n, int64_t m);
+inline int alt_for(int slots, int mode, int gpu_rule, bool batch, int64_t n, int64_t m, const Layout &ly, const Regions &rg) {
+  if (slots < 2 || gpu_rule) return 0;
+  if (mode == 0) return !batch && mark_test_for(n, m) ? 1 : 0;
+  return mode == 2 && rg.wide_items > 0 && ly.hub_min <= (int64_t(1) << 29) && ly.hub_chunk <= (int64_t(1) << 29) ? 1 : 0;
+}
+
 // Sort key of a vertex in the plan (regions in order, region 6 by degree descending);
 // key_isolated for degree 0. Shared by the device plan kernel and the host summary.
 __host__ __device__ inline uint32_t plan_key(int64_t deg, const Layout &ly) {
@@ -81,6 +120,8 @@ __host__ __device__ inline uint32_t plan_key(int64_t deg, const Layout &ly) {
 }
 __host__ __device__ inline int key_region(uint32_t key) { return key < 6 ? int(key) : REG_LANE; }
 
+// The buffer of a launch's RunState (rak_device.cuh); RunStateHost is its head, which the host reads back.
+constexpr size_t RUN_STATE_BYTES = 256;
 struct RunStateHost {
   unsigned int bar, abort, error, iterations;
   unsigned long long asym;
@@ -133,6 +174,7 @@ struct LpaArgs {
   // synchronous modes: k_symmetry has run before the launch, so iterations may find their active set by
   // looking for neighbours that moved (lpa_run); all_flags: every vertex starts affected
   int pull, all_flags;
+  int alt;    // the other kernel of the mode (alt_for)
 };
 
 // Whether a run asks k_symmetry for that: it needs a second iteration to gain anything.
@@ -161,7 +203,7 @@ inline int default_label_order(int mode, int slots) { return mode == MODE_ASYNC 
 // STAT_PHASE: how the iteration treated the frontier (bit 0: its moves marked no neighbours; bit 1:
 // it processed every vertex), written by the asynchronous single-graph kernel.
 enum Stat { STAT_CHANGED = 0, STAT_EDGES = 1, STAT_PROCESSED = 2, STAT_HUBS_MOVED = 3, STAT_MOVED_EDGES = 4, STAT_WORK = 5,
-            STAT_PHASE = 6 };
+            STAT_PHASE = 6, STAT_WIDE = 7 };
 constexpr int STATS_STRIDE = 8;
 
 // Persistent cooperative launch of all iterations; grid chosen from occupancy. `batch` selects the
@@ -172,7 +214,10 @@ cudaError_t launch_lpa(const LpaArgs &a, int slots, int mode, bool off64, cudaSt
 template <int S>
 cudaError_t launch_lpa_slots(const LpaArgs &a, int mode, bool off64, bool batch, cudaStream_t st, int *grid_out);
 template <int S>
-cudaError_t resolve_lpa_slots(int mode, bool off64, bool unit, bool batch, bool stage, const void **fn, int *per_sm);
+cudaError_t resolve_lpa_slots(int mode, bool off64, bool unit, bool batch, bool stage, bool alt, const void **fn, int *per_sm);
+// The asynchronous kernel that keeps its pace (rak_lpa_async.cuh; rak_lpa_async_s*.cu).
+template <int S>
+const void *async_kernel(bool off64, bool unit, bool batch);
 // Whether neighbour marking reads each flag (through L1) before storing it. Measured on B200 with
 // the read through L1, test on / off, νMG8 and νBM: R-MAT scale 24 ef 32 (16.8 M vertices) 31.3 /
 // 36.9 ms and 23.1 / 32.2 ms; R-MAT scale 27 ef 16 (134 M) 128.0 / 135.6 ms and 125.6 / 139.5 ms --
@@ -193,7 +238,7 @@ inline int mark_test_for_batch(int64_t n, int64_t m, int64_t graphs) {
 cudaError_t launch_symmetry(const void *off, bool off64, const uint32_t *tgt, int64_t n, int64_t m, const uint32_t *gid,
                             const int64_t *vbase, void *rs, cudaStream_t st);
 // Loads and resolves the kernel a run will launch (outside its timed region).
-cudaError_t prepare_lpa(int slots, int mode, bool off64, bool unit, bool batch, bool stage);
+cudaError_t prepare_lpa(int slots, int mode, bool off64, bool unit, bool batch, bool stage, bool alt);
 
 // Plan and utility kernels (rak_kernels.cu).
 cudaError_t launch_validate(const void *off, bool off64, const uint32_t *tgt, int64_t n, int64_t m,

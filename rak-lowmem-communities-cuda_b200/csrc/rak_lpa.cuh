@@ -149,10 +149,9 @@ __device__ __forceinline__ float edge_w(const float *wt, int64_t e) {
 // Software-pipelined in three stages of two edges: while one stage's labels are accumulated, the next
 // stage's labels and the targets (and weights) of the one after are on their way. Positions past the
 // end are given the target u itself, which the self-loop rule skips. Labels are read with plain loads:
-// they change during the launch. Before (two stages of four edges, labels waited for) -> now, with the
-// whole-number sketch below, measured on B200: R-MAT scale 24 ef 16 11.3 -> 10.5 ms, scale 22 3.37 -> 3.15
-// ms, scale 20 2.86 -> 2.52 ms, scale 22 ef 32 weighted 9.7 -> 9.2 ms; lattice 2047x2049 1.13 -> 1.15 ms,
-// SBM 2 M vertices 1.29 -> 1.33 ms. Three edges a stage: scale 20 2.27 ms, lattice 1.19 ms.
+// they change during the launch. Two stages of four edges, whose labels were waited for -> this, with the
+// whole-number sketch below, asynchronous runs measured on B200: R-MAT scale 24 ef 16 11.3 -> 10.5 ms, scale 22
+// 3.37 -> 3.15 ms, scale 22 ef 32 weighted 9.7 -> 9.2 ms.
 template <bool UNIT, class ACC>
 __device__ __forceinline__ void scan_edges(ACC &&acc, uint32_t u, int64_t e, int64_t ee, int st, const uint32_t *tgt,
                                            const float *wt, const uint32_t *vin, uint32_t base) {
@@ -668,7 +667,7 @@ __device__ __forceinline__ bool move_rule(float w, uint32_t c, uint32_t d, bool 
 template <int S, int RULE>
 __device__ __forceinline__ void choose(const LpaArgs &a, const Sketch<S> &sk, uint32_t u_local, int it, uint32_t &c,
                                        float &w) {
-  if constexpr (S > 1 && RULE == RULE_CPU) {
+  if constexpr (S > 1 && RULE != RULE_GPU) {
     const int l = a.start_iter + it;
     if (l < a.tie_until) {
       sk_choose_hashed<S>(sk, u_local, uint32_t(l), c, w);
@@ -739,8 +738,8 @@ __device__ __forceinline__ bool lane_active(const LpaArgs &a, const G_<O> &g, ui
 
 template <int MODE, class O, bool BATCH>
 __device__ __forceinline__ int lane_collect(const LpaArgs &a, const Regions &rg, const G_<O> &g, int64_t local,
-                                            const uint32_t *vin, uint32_t *vout, const uint8_t *fin, uint32_t *q, int qn,
-                                            Phase ph) {
+                                            const uint32_t *vin, uint32_t *vout, const uint8_t *fin, uint8_t *fout,
+                                            uint32_t *q, int qn, Phase ph) {
   const int lane = threadIdx.x & 31;
   const int64_t idx = local * 32 + lane;
   bool act = false;
@@ -749,7 +748,10 @@ __device__ __forceinline__ int lane_collect(const LpaArgs &a, const Regions &rg,
     u = __ldg(a.order + rg.vbegin[REG_LANE] + idx);
     act = lane_active<O, BATCH>(a, g, u, fin, ph);
     if constexpr (MODE != MODE_ASYNC)
-      if (!act) vout[u] = vin[u];
+      if (!act) {
+        vout[u] = vin[u];
+        if (ph.pull_out) fout[u] = 0;
+      }
   }
   const unsigned m = __ballot_sync(FULL, act);
   if (act) q[qn + __popc(m & ((1u << lane) - 1u))] = u;
@@ -773,7 +775,7 @@ __device__ __forceinline__ bool lane_close(const LpaArgs &a, const Sketch<S> &sk
     if (moved) vout[u] = c;
   } else {
     vout[u] = moved ? c : d;
-    if (moved && ph.pull_out) fout[u] = 1;
+    if (ph.pull_out) fout[u] = moved ? 1 : 0;
   }
   if (moved) {
     cnt.changed += 1;
@@ -827,7 +829,9 @@ __device__ __forceinline__ GroupVertex group_open(const LpaArgs &a, const Region
     v.active = !graph_of<BATCH>(a, v.u, v.gi, v.base) && (ph.pull_in || ph.all || fin[v.u] != 0);
     if (v.active) { v.eb = int64_t(__ldg(g.off + v.u)); v.ee = int64_t(__ldg(g.off + v.u + 1)); }
   }
-  if (ph.pull_in) v.active = group_pull(v.active, v.u, v.eb, v.ee, s, G, grp, g.tgt, fin, v.base);
+  if (ph.pull_in)
+    v.active = G == 1 ? v.active && lane_pull(v.u, v.eb, v.ee, g.tgt, fin, v.base)
+                      : group_pull(v.active, v.u, v.eb, v.ee, s, G, grp, g.tgt, fin, v.base);
   return v;
 }
 // Merges the group's sketches, chooses and moves; true on every lane of the group if it moved.
@@ -850,7 +854,7 @@ __device__ __forceinline__ bool group_close(const LpaArgs &a, Sketch<S> &sk, con
       if (moved) vout[v.u] = c;
     } else {
       vout[v.u] = moved ? c : v.d;
-      if (moved && ph.pull_out) fout[v.u] = 1;
+      if (ph.pull_out) fout[v.u] = moved ? 1 : 0;
     }
     if (moved) { cnt.changed += 1; cnt.moved_edges += (unsigned long long)(v.ee - v.eb); count_move<BATCH>(a, v.gi, it); }
   }
@@ -958,7 +962,10 @@ __device__ __forceinline__ void hub_close(const LpaArgs &a, Sketch<S> &sk, const
   if (lane == 0) a.hub_arrive[k.h] = 0;
   const uint32_t d = vin[k.u];
   if (!k.active) {
-    if (MODE != MODE_ASYNC && lane == 0) vout[k.u] = d;
+    if (MODE != MODE_ASYNC && lane == 0) {
+      vout[k.u] = d;
+      if (ph.pull_out) fout[k.u] = 0;
+    }
     return;
   }
   Sketch<S> acc;
@@ -984,7 +991,7 @@ __device__ __forceinline__ void hub_close(const LpaArgs &a, Sketch<S> &sk, const
       if (moved) vout[k.u] = c;
     } else {
       vout[k.u] = moved ? c : d;
-      if (moved && ph.pull_out) fout[k.u] = 1;
+      if (ph.pull_out) fout[k.u] = moved ? 1 : 0;
     }
     if (moved) {
       cnt.changed += 1;
@@ -1014,7 +1021,7 @@ __device__ __forceinline__ void hub_item(const LpaArgs &a, const Regions &rg, co
     const bool moved = k.active && move_rule<S, RULE>(w, c, d, pickless);
     if (lane == 0) {
       vout[k.u] = moved ? c : d;
-      if (moved && ph.pull_out) fout[k.u] = 1;
+      if (ph.pull_out) fout[k.u] = moved ? 1 : 0;
       if (k.active) { cnt.processed += 1; cnt.edges += (unsigned long long)(k.ee - k.eb); }
       if (moved) { cnt.changed += 1; cnt.moved_edges += (unsigned long long)(k.ee - k.eb); count_move<BATCH>(a, k.gi, it); }
     }
@@ -1035,20 +1042,183 @@ __device__ __forceinline__ void hub_item(const LpaArgs &a, const Regions &rg, co
   }
 }
 
+// ---- wide items: 32 sketches scanned by a whole block, a thread for every slot -------------------
+//
+// A warp item scans 32 edge sequences (chains), one per lane. A chain cannot be split -- each edge meets
+// the sketch the ones before it left -- so its warp's pace bounds the iteration: about 1000 cycles a step
+// on a busy SM (measured; 2048 steps for a degree of 65536), and on graphs of a few million edges that is
+// most of the iteration (R-MAT scale 20: 1.0 of 1.03 ms; the edges alone take 0.1 ms). Here the block's 256
+// threads take the same 32 chains, S threads a chain and one slot each: a step is a shuffle, a compare and
+// two votes instead of a pass over S slots, the S threads load S edges of the chain at once, and the next
+// edges' labels are gathered meanwhile. The sketches go through shared memory to the block's first warp,
+// which merges, chooses and moves exactly as for a warp item; marking is spread over the block. Bit for
+// bit the same sketches. It costs more instructions per edge, so only chains too long for the graph are
+// scanned this way (Regions::wide_len). Measured on B200, split runs, without -> with: R-MAT scale 12 ef 16
+// 0.42 -> 0.31 ms, scale 16 1.5 -> 1.03 ms, scale 18 2.7 -> 2.3 ms, scale 20 10.9 -> 6.5 ms, scale 20 ef 32
+// weighted 13.7 -> 9.6 ms.
+template <int S>
+struct WideShared {
+  long long item;
+  int64_t eb[32], ee[32];   // chain: edges eb, eb + st, ... < ee of vertex u
+  uint32_t u[32], base[32];
+  int st;
+  unsigned live, moved;     // chains to scan; chains whose vertex moved
+  uint32_t k[32 * S];
+  float w[32 * S];
+};
+template <int S, int MODE>
+__host__ __device__ constexpr bool has_wide() { return MODE == MODE_SPLIT && S > 1; }
+
+template <int S, bool UNIT>
+__device__ __forceinline__ void scan_slots(WideShared<S> &ws, const uint32_t *tgt, const float *wt, const uint32_t *vin) {
+  const int slot = threadIdx.x & (S - 1), shift = threadIdx.x & 31 & ~(S - 1), st = ws.st;
+  constexpr unsigned GM = (1u << S) - 1u;   // the chain's S threads, from bit `shift` of a vote on
+  for (int c = threadIdx.x / S; c < 32; c += 256 / S) {   // the same trip count on every lane of a warp
+    const uint32_t u = ws.u[c], base = ws.base[c];
+    const int64_t e = ws.eb[c];
+    const int len = (ws.live >> c) & 1u ? int((ws.ee[c] - e + st - 1) / st) : 0;
+    const int most = __reduce_max_sync(FULL, len);
+    const uint32_t *tp = tgt + e + int64_t(slot) * st;
+    const float *wp = UNIT ? nullptr : wt + e + int64_t(slot) * st;
+    const int64_t hop = int64_t(S) * st;
+    uint32_t k = NONE, num = 0u, low = 0u;   // unit weights: the weight is num - low, low shared by the chain
+    float w = 0.0f;
+    // this thread's edge of the current S steps (its label gathered), and of the next S
+    uint32_t t0 = slot < len ? base + ld_edge(tp) : u, t1 = S + slot < len ? base + ld_edge(tp + hop) : u;
+    float w0 = slot < len ? edge_w<UNIT>(wp, 0) : 0.0f, w1 = S + slot < len ? edge_w<UNIT>(wp, hop) : 0.0f;
+    uint32_t c0 = t0 != u ? ld_label(vin + t0) : NONE;
+    for (int done = 0; done < most; done += S) {
+      const uint32_t c1 = t1 != u ? ld_label(vin + t1) : NONE;
+      const bool far = done + 2 * S + slot < len;
+      const uint32_t t2 = far ? base + ld_edge(tp + 2 * hop) : u;
+      const float w2 = far ? edge_w<UNIT>(wp, 2 * hop) : 0.0f;
+      const unsigned has = __ballot_sync(FULL, t0 != u) >> shift;   // self-loops and ends take no step
+#pragma unroll
+      for (int i = 0; i < S; ++i) {
+        const uint32_t cc = __shfl_sync(FULL, c0, i, S);
+        const float x = UNIT ? 1.0f : __shfl_sync(FULL, w0, i, S);
+        const bool on = (has >> i) & 1u;
+        const bool hit = on && k == cc;
+        // votes by every lane, outside any condition (both votes side by side measured 10-15% slower)
+        const unsigned hits = (__ballot_sync(FULL, hit) >> shift) & GM;
+        const bool miss = on && hits == 0u;
+        const unsigned open = (__ballot_sync(FULL, miss && (UNIT ? num == low : w == 0.0f)) >> shift) & GM;
+        const bool take = open != 0u && slot == 31 - __clz(int(open));   // the last free slot
+        if constexpr (UNIT) {
+          if (hit) num += 1u;
+          if (take) { k = cc; num = low + 1u; }
+          if (miss && open == 0u) low += 1u;
+        } else {
+          if (hit) w = __fadd_rn(w, x);
+          if (take) { k = cc; w = x; }
+          if (miss && open == 0u) w = fmaxf(__fsub_rn(w, x), 0.0f);
+        }
+      }
+      t0 = t1; c0 = c1; w0 = w1; t1 = t2; w1 = w2;
+      tp += hop;
+      if constexpr (!UNIT) wp += hop;
+    }
+    ws.k[c * S + slot] = k;
+    ws.w[c * S + slot] = UNIT ? float(num - low) : w;
+  }
+}
+
+// Whether item `local` of region 0 or 1 is a wide one where only their longest are (!Regions::wide_all).
+template <class O>
+__device__ __forceinline__ bool long_item(const LpaArgs &a, const Regions &rg, const G_<O> &g, int r, int64_t local) {
+  int64_t edges = a.hub_chunk;
+  if (r != REG_HUB) {
+    const uint32_t u = __ldg(a.order + rg.vbegin[r] + local);
+    edges = int64_t(__ldg(g.off + u + 1)) - int64_t(__ldg(g.off + u));
+  }
+  return edges > 32 * int64_t(rg.wide_len);
+}
+
+// The iteration's wide items, taken by whole blocks from a counter of their own. A function of its own,
+// not inlined: its registers would crowd the warp items' loops (inlined: lattice 2047x2049 1.16 -> 1.36 ms).
+template <int S, int MODE, class O, bool UNIT, bool BATCH>
+__device__ __noinline__ Counters wide_items(const LpaArgs &a, const Regions &rg, int it, bool pickless,
+                                            const uint32_t *vin, uint32_t *vout, uint8_t *fin, uint8_t *fout, Phase ph,
+                                            WideShared<S> &ws) {
+  const G_<O> g{static_cast<const O *>(a.off), a.tgt, a.wt};
+  const int lane = threadIdx.x & 31;
+  Counters cnt{0, 0, 0, 0};
+  for (int64_t taken = 0; taken <= rg.wide_items; ++taken) {
+    __syncthreads();   // ws of the item before is no longer read
+    if (threadIdx.x == 0) ws.item = (long long)atomicAdd(a.stats + STATS_STRIDE * it + STAT_WIDE, 1ull);
+    __syncthreads();
+    const int64_t item = ws.item;
+    if (item >= rg.wide_items) break;
+    int r = 0;
+    while (r < REG_LANE && item >= rg.ibegin[r + 1]) ++r;
+    const int64_t local = item - rg.ibegin[r];   // region 6: a batch of 32 vertices
+    if (!rg.wide_all && !long_item(a, rg, g, r, local)) continue;
+    GroupVertex v;
+    HubChunk k;
+    if (threadIdx.x < 32) {
+      const int G = region_group(r), s = lane & (G - 1);
+      if (r == REG_HUB) {
+        k = hub_open<MODE, O, BATCH>(a, rg, g, local, it, fin, ph);
+        ws.u[lane] = k.u; ws.base[lane] = k.base; ws.eb[lane] = k.cb + lane; ws.ee[lane] = k.ce;
+      } else {
+        v = group_open<O, BATCH>(a, rg, g, r, local, vin, fin, ph);
+        ws.u[lane] = v.u; ws.base[lane] = v.base; ws.eb[lane] = v.eb + s; ws.ee[lane] = v.ee;
+      }
+      const unsigned live = __ballot_sync(FULL, r == REG_HUB ? k.active : v.active);
+      if (lane == 0) { ws.st = G; ws.live = live; ws.moved = 0u; }
+    }
+    __syncthreads();
+    if (ws.live) scan_slots<S, UNIT>(ws, g.tgt, g.wt, vin);
+    __syncthreads();
+    if (threadIdx.x < 32) {
+      Sketch<S> sk;
+      sk_clear<S>(sk);
+      if ((ws.live >> lane) & 1u) {
+#pragma unroll
+        for (int i = 0; i < S; ++i) { sk.k[i] = ws.k[lane * S + i]; sk.w[i] = ws.w[lane * S + i]; }
+      }
+      if (r == REG_HUB) {
+        hub_close<S, MODE, BATCH, RULE_CPU>(a, sk, k, NONE, local, it, pickless, vin, vout, fout, cnt, ph);
+      } else {
+        const unsigned moved = __ballot_sync(FULL, group_close<S, MODE, BATCH, RULE_CPU>(a, sk, v, r, it, pickless, vout, fin, fout, cnt, ph));
+        if (lane == 0) ws.moved = moved;
+      }
+    }
+    if (ph.nomark || ph.pull_out || r == REG_HUB) continue;
+    __syncthreads();
+    const int c = threadIdx.x >> 3;   // eight threads mark a chain's edges
+    if ((ws.moved >> c) & 1u)
+      mark_item<S>(a, ws.u[c], ws.eb[c] + int64_t(threadIdx.x & 7) * ws.st, ws.ee[c], 8 * ws.st, g.tgt, fout, ws.base[c]);
+  }
+  return cnt;
+}
+
 // The rule set of a work item: the exact synchronous mode follows the CPU rules; the split-layout
 // modes (asynchronous and synchronous split) either, per launch (a.gpu_rule).
 #define RAK_BY_RULE(F, ARGS)                                                            \
   do {                                                                                 \
     if constexpr (MODE != MODE_SYNC) {                                                 \
       if (a.gpu_rule) F<S, MODE, O, UNIT, BATCH, RULE_GPU> ARGS;                       \
-      else F<S, MODE, O, UNIT, BATCH, RULE_CPU> ARGS;                                  \
+      else F<S, MODE, O, UNIT, BATCH, RULE_CPU> ARGS;                       \
     } else {                                                                           \
       F<S, MODE, O, UNIT, BATCH, RULE_CPU> ARGS;                                       \
     }                                                                                  \
   } while (0)
 
-template <int S, int MODE, class O, bool UNIT, bool BATCH>
-__global__ void __launch_bounds__(256, RAK_MIN_BLOCKS) lpa_run(const LpaArgs a) {
+// Whether iteration it + 1 records its movers for the one after it: when the vertices that moved in
+// iteration it hold a quarter of the edges or more (in the first iteration: when every vertex starts
+// affected). Every block reads the same counter after the barrier, so all agree; the choice changes what
+// the flags hold, not the result.
+__device__ __forceinline__ bool pulls_next(const LpaArgs &a, int it, bool can_pull) {
+  return can_pull && it + 2 < a.iters &&
+         __ldcg(a.stats + STATS_STRIDE * it + STAT_MOVED_EDGES) * 4ull >= (unsigned long long)a.m;
+}
+
+// WIDE: the launch has wide items. Launches without any take a kernel that does not hold their code and
+// shared memory (one kernel for both: R-MAT scale 24 ef 16 split 50.7 -> 52.4 ms, lattice 2047x2049 1.16 -> 1.24
+// ms). Asynchronous runs take this kernel only where their result does not show its pace (rak_lpa_async.cuh).
+template <int S, int MODE, class O, bool UNIT, bool BATCH, bool WIDE>
+__global__ void __launch_bounds__(256, RAK_MIN_BLOCKS) lpa_run(const __grid_constant__ LpaArgs a) {
   const G_<O> g{static_cast<const O *>(a.off), a.tgt, a.wt};
   RunState *rs = static_cast<RunState *>(a.rs);
   const int lane = threadIdx.x & 31;
@@ -1057,6 +1227,7 @@ __global__ void __launch_bounds__(256, RAK_MIN_BLOCKS) lpa_run(const LpaArgs a) 
   __shared__ unsigned long long blk[4];
   __shared__ Regions rg;  // copied once: indexed by region at run time
   __shared__ uint32_t lq[8][64];  // per-warp queue of active one-lane vertices
+  __shared__ WideShared<WIDE ? S : 1> ws;
   if (threadIdx.x == 0) rg = a.rg;
   // staged edge tiles (not in the exact synchronous mode, which shuffles edges in order instead)
   StageCtx sc{};
@@ -1090,6 +1261,7 @@ __global__ void __launch_bounds__(256, RAK_MIN_BLOCKS) lpa_run(const LpaArgs a) 
   // counter, which every block reads after the barrier, so all blocks agree.
   Phase ph{false, false, false, false};
   const bool can_pull = MODE != MODE_ASYNC && a.pull != 0 && __ldcg(&rs->asym) == 0ull;
+  bool next_out = false;   // whether the next iteration records its movers (Phase::pull_out)
   for (int it = 0; it < a.iters; ++it) {
     if (threadIdx.x < 4) blk[threadIdx.x] = 0;
     if constexpr (MODE == MODE_ASYNC && !BATCH) {
@@ -1100,13 +1272,8 @@ __global__ void __launch_bounds__(256, RAK_MIN_BLOCKS) lpa_run(const LpaArgs a) 
         a.stats[STATS_STRIDE * it + STAT_PHASE] = (ph.all ? 2ull : 0ull) | (ph.nomark ? 1ull : 0ull);
     }
     if constexpr (MODE != MODE_ASYNC) {
-      // Pull when the previous iteration's moved vertices hold a quarter of the edges or more (in the
-      // first iteration: when every vertex starts affected). Every block reads the same counter after
-      // the barrier, so all blocks agree; the choice changes what the next iteration reads, not its result.
       ph.pull_in = ph.pull_out;
-      ph.pull_out = can_pull && it + 1 < a.iters &&
-                    (it == 0 ? a.all_flags != 0
-                             : __ldcg(a.stats + STATS_STRIDE * (it - 1) + STAT_MOVED_EDGES) * 4ull >= (unsigned long long)a.m);
+      ph.pull_out = it == 0 ? can_pull && a.iters > 1 && a.all_flags != 0 : next_out;
     }
     __syncthreads();
     const int l = a.start_iter + it;
@@ -1121,19 +1288,27 @@ __global__ void __launch_bounds__(256, RAK_MIN_BLOCKS) lpa_run(const LpaArgs a) 
     unsigned long long *work = a.stats + STATS_STRIDE * it + STAT_WORK;
     uint32_t *q = lq[threadIdx.x >> 5];
     int qn = 0;
+    int64_t item0 = 0;     // the first warp item: after the wide ones where these are all of the first
+    bool skip_long = false;
+    if constexpr (WIDE) {
+      cnt = wide_items<S, MODE, O, UNIT, BATCH>(a, rg, it, pickless, vin, vout, fin, fout, ph, ws);
+      if (rg.wide_all) item0 = rg.ibegin[REG_LANE] + rg.wide_lanes / rg.lane_item;
+      else skip_long = true;
+    }
     for (;;) {
       unsigned long long got = 0;
       if (lane == 0) got = atomicAdd(work, 1ull);
-      const int64_t item = int64_t(__shfl_sync(FULL, got, 0));
+      const int64_t item = item0 + int64_t(__shfl_sync(FULL, got, 0));
       if (item >= total) break;
       int r = 0;
       while (item >= rg.ibegin[r + 1]) ++r;
       const int64_t local = item - rg.ibegin[r];
+      if (WIDE && skip_long && r <= 1 && long_item(a, rg, g, r, local)) continue;
       if (r == REG_LANE) {
         for (int64_t sb = 0; sb < rg.lane_item; ++sb) {
           const int64_t sub = local * rg.lane_item + sb;
           if (sub * 32 >= rg.vcount[REG_LANE]) break;
-          qn = lane_collect<MODE, O, BATCH>(a, rg, g, sub, vin, vout, fin, q, qn, ph);
+          qn = lane_collect<MODE, O, BATCH>(a, rg, g, sub, vin, vout, fin, fout, q, qn, ph);
           if (qn >= 32) {
             RAK_BY_RULE(lane_batch, (a, g, q, 32, it, pickless, vin, vout, fin, fout, cnt, ph));
             __syncwarp();
@@ -1208,6 +1383,7 @@ __global__ void __launch_bounds__(256, RAK_MIN_BLOCKS) lpa_run(const LpaArgs a) 
       run = warp_sum(run);
       if (lane == 0 && run) atomicAdd(a.running + it, run);
       if constexpr (MODE != MODE_ASYNC) {
+        next_out = pulls_next(a, it, can_pull);
         uint4 *f4 = reinterpret_cast<uint4 *>(fin);
         const int64_t n16 = a.n >> 4;
         for (int64_t i = tid; i < n16; i += nt) f4[i] = make_uint4(0, 0, 0, 0);
@@ -1225,6 +1401,10 @@ __global__ void __launch_bounds__(256, RAK_MIN_BLOCKS) lpa_run(const LpaArgs a) 
       return;
     }
     if constexpr (MODE != MODE_ASYNC) {
+      next_out = pulls_next(a, it, can_pull);
+      // Every vertex with an edge writes its flag in an iteration that records movers: nothing to clear,
+      // and nothing after the barrier above to wait for unless this one marked split vertices' neighbours.
+      if (next_out && ph.pull_out) continue;
       // The flags just read become next iteration's output: clear them.
       const int64_t tid = int64_t(blockIdx.x) * blockDim.x + threadIdx.x, nt = int64_t(gridDim.x) * blockDim.x;
       uint4 *f4 = reinterpret_cast<uint4 *>(fin);
@@ -1247,12 +1427,23 @@ inline size_t lpa_dynamic_smem(int mode, bool unit, bool stage) {
 // device). The first query of an instantiation loads its module (CUDA loads modules lazily, which
 // can take a millisecond), so runs resolve before their timed region (prepare_lpa).
 template <int S>
-cudaError_t resolve_lpa_slots(int mode, bool off64, bool unit, bool batch, bool stage, const void **fn_out,
+cudaError_t resolve_lpa_slots(int mode, bool off64, bool unit, bool batch, bool stage, bool alt, const void **fn_out,
                               int *per_sm_out) {
   const void *fn = nullptr;
 #define RAK_PICK(M, O, U, B)                                                          \
-  if (mode == M && off64 == (sizeof(O) == 8) && unit == U && batch == B)             \
-    fn = reinterpret_cast<const void *>(&lpa_run<S, M, O, U, B>);
+  if (mode == M && off64 == (sizeof(O) == 8) && unit == U && batch == B) {           \
+    if constexpr (M == MODE_ASYNC) {                                                  \
+      fn = async_kernel<S>(off64, unit, batch);                                        \
+      if constexpr (S > 1 && !B) {                                                    \
+        if (alt) fn = reinterpret_cast<const void *>(&lpa_run<S, M, O, U, B, false>); \
+      }                                                                               \
+    } else {                                                                          \
+      fn = reinterpret_cast<const void *>(&lpa_run<S, M, O, U, B, false>);            \
+      if constexpr (has_wide<S, M>()) {                                               \
+        if (alt) fn = reinterpret_cast<const void *>(&lpa_run<S, M, O, U, B, true>);  \
+      }                                                                               \
+    }                                                                                 \
+  }
 #define RAK_PICK_MODE(M)                                                             \
   RAK_PICK(M, int32_t, false, false) RAK_PICK(M, int32_t, true, false)                \
   RAK_PICK(M, int64_t, false, false) RAK_PICK(M, int64_t, true, false)                \
@@ -1292,13 +1483,14 @@ template <int S>
 cudaError_t launch_lpa_slots(const LpaArgs &a, int mode, bool off64, bool batch, cudaStream_t st, int *grid_out) {
   const void *fn = nullptr;
   int per_sm = 0, dev = 0, sms = 0;
-  cudaError_t e = resolve_lpa_slots<S>(mode, off64, a.wt == nullptr, batch, a.stage != 0, &fn, &per_sm);
+  cudaError_t e = resolve_lpa_slots<S>(mode, off64, a.wt == nullptr, batch, a.stage != 0, a.alt != 0, &fn, &per_sm);
   if (e != cudaSuccess) return e;
   if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
   if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
   const int64_t warps_needed = a.rg.ibegin[NREG] > 0 ? a.rg.ibegin[NREG] : 1;
   int64_t grid = int64_t(per_sm) * sms;
-  const int64_t want = (warps_needed + 7) / 8;
+  int64_t want = (warps_needed + 7) / 8;
+  if (mode == MODE_SPLIT && a.alt && a.rg.wide_items > want) want = a.rg.wide_items;   // a block each
   if (want < grid) grid = want;
   if (a.grid_cap > 0 && grid > a.grid_cap) grid = a.grid_cap;
   if (grid < 1) grid = 1;

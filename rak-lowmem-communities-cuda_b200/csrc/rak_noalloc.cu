@@ -244,6 +244,7 @@ extern "C" rak_status rak_lowmem_cuda_noalloc(int device, void *stream, const ra
       it += region_items(r, cnt[r], nchunks, rg.lane_item);
     }
     rg.ibegin[NREG] = it;
+    set_wide(&rg, h, ly, g->m);
   }
 
   // ---- run buffers ---------------------------------------------------------------------------------
@@ -257,7 +258,7 @@ extern "C" rak_status rak_lowmem_cuda_noalloc(int device, void *stream, const ra
   uint32_t *skk = cv.take<uint32_t>(size_t(nchunks > 0 ? nchunks : 1) * size_t(slots));
   float *skw = cv.take<float>(size_t(nchunks > 0 ? nchunks : 1) * size_t(slots));
   unsigned long long *stats = cv.take<unsigned long long>(size_t(it_slots) * STATS_STRIDE);
-  RunStateHost *rs = cv.take<RunStateHost>(1);
+  unsigned char *rs = cv.take<unsigned char>(RUN_STATE_BYTES);
   if (cv.need > RAK_NOALLOC_SCRATCH_BYTES) { rr->peak_device_bytes = cv.need; return RAK_ERR_OUT_OF_MEMORY; }
   if (nhub > 0) {
     k_chunk_owner<<<blocks_for(nhub), 256, 0, st>>>(first, nhub, chunk_hub);
@@ -267,10 +268,11 @@ extern "C" rak_status rak_lowmem_cuda_noalloc(int device, void *stream, const ra
   NA_TRY(cudaMemsetAsync(claim, 0, size_t(nhub > 0 ? nhub : 1) * 4, st));
   NA_TRY(cudaMemsetAsync(moved, 0xFF, size_t(nhub > 0 ? nhub : 1) * 4, st));
   NA_TRY(cudaMemsetAsync(stats, 0, size_t(it_slots) * STATS_STRIDE * 8, st));
-  NA_TRY(cudaMemsetAsync(rs, 0, sizeof(RunStateHost), st));
+  NA_TRY(cudaMemsetAsync(rs, 0, RUN_STATE_BYTES, st));
   // the kernel's code is loaded (CUDA loads modules lazily) before the timed part
   const bool stage = (o->edge_staging <= 0 ? DEFAULT_EDGE_STAGING : o->edge_staging) == 1;
-  if (iters > 0) NA_TRY(prepare_lpa(slots, mode, off64, g->weights == nullptr, false, stage));
+  if (iters > 0) NA_TRY(prepare_lpa(slots, mode, off64, g->weights == nullptr, false, stage,
+                                   alt_for(slots, mode, o->sketch_rule == 2, false, n, g->m, ly, rg)));
   const auto t1 = std::chrono::steady_clock::now();
   if (ref_labels) NA_TRY(launch_init_mapped(membership, q, ref_pos, n, st));
   else NA_TRY(launch_init(membership, vcom1, q, n, st));
@@ -289,6 +291,7 @@ extern "C" rak_status rak_lowmem_cuda_noalloc(int device, void *stream, const ra
   a.mark_test = mark_test_for(n, g->m);
   // rule sets as in rak_lowmem_cuda: the CPU rules unless sketch_rule asks for the GPU ones
   a.gpu_rule = mode != RAK_MODE_SYNC && o->sketch_rule == 2;
+  a.alt = alt_for(slots, mode, a.gpu_rule, false, n, g->m, ly, rg);
   // ties as in rak_lowmem_cuda: hashed during the first iterations of asynchronous runs
   const int tie = o->tie_break <= 0 ? (mode == RAK_MODE_ASYNC && !a.gpu_rule ? 2 : 1) : o->tie_break;
   a.tie_until = tie == 2 ? (o->tie_iterations > 0 ? o->tie_iterations : DEFAULT_TIE_ITERATIONS) : 0;
