@@ -16,6 +16,7 @@
 #include <condition_variable>
 #include <cstring>
 #include <deque>
+#include <initializer_list>
 #include <limits>
 #include <memory>
 #include <mutex>
@@ -35,6 +36,20 @@ struct rak_ctx {
   std::string err;
   cudaMemPool_t pool = nullptr;  // one-shot runs allocate here while keep > 0 (rak_ctx_set_memory_keep)
   uint64_t keep = 0;
+  // Kept for the context's next call, freed with it: device scratch of calls that need no more than
+  // SCRATCH_KEEP (a call waits for its work before it returns, so the next one may reuse it on any
+  // stream), and timing events not in use.
+  static constexpr size_t SCRATCH_KEEP = size_t(64) << 20;
+  void *scratch = nullptr;
+  size_t scratch_bytes = 0;
+  std::vector<cudaEvent_t> events;
+  rak_ctx() = default;
+  rak_ctx(const rak_ctx &) = delete;
+  rak_ctx &operator=(const rak_ctx &) = delete;
+  ~rak_ctx() {
+    for (cudaEvent_t e : events) cudaEventDestroy(e);
+    if (scratch) cudaFree(scratch);
+  }
 };
 
 namespace rak_host_detail {
@@ -49,9 +64,24 @@ struct Tracker {
 // Where this thread's device allocations come from: cudaMalloc (no pool), or stream-ordered from
 // a memory pool on a stream (PoolScope). The server's launch slots use their own pools, so that
 // growing a slot's buffers never waits for the whole device (cudaFree does).
+// An arena is one block that a call's buffers are carved from, in order, never given back before the call
+// ends (ArenaScope): a call on a new graph otherwise maps and unmaps some twenty buffers, and on a busy
+// host each of those takes up to milliseconds.
+struct Arena {
+  char *base = nullptr;
+  size_t size = 0, used = 0;
+  static size_t rounded(size_t b) { return ((b ? b : 16) + 255) / 256 * 256; }
+  bool fits(size_t b) const { return base && used + rounded(b) <= size; }
+  void *take(size_t b) {
+    void *p = base + used;
+    used += rounded(b);
+    return p;
+  }
+};
 struct PoolTarget {
   cudaMemPool_t pool = nullptr;
   cudaStream_t stream = nullptr;
+  Arena *arena = nullptr;
 };
 inline PoolTarget &thread_pool() {
   static thread_local PoolTarget t;
@@ -59,7 +89,7 @@ inline PoolTarget &thread_pool() {
 }
 struct PoolScope {
   PoolTarget saved;
-  PoolScope(cudaMemPool_t pool, cudaStream_t stream) : saved(thread_pool()) { thread_pool() = {pool, stream}; }
+  PoolScope(cudaMemPool_t pool, cudaStream_t stream) : saved(thread_pool()) { thread_pool() = {pool, stream, nullptr}; }
   ~PoolScope() { thread_pool() = saved; }
 };
 
@@ -81,21 +111,29 @@ struct DevBuf {
   size_t bytes = 0;
   Tracker *t = nullptr;
   bool pooled = false;
+  bool carved = false;        // from an arena
   cudaStream_t fs = nullptr;  // stream a pooled buffer is freed on
   DevBuf() = default;
   DevBuf(const DevBuf &) = delete;
   DevBuf &operator=(const DevBuf &) = delete;
   ~DevBuf() { release(); }
   void release() {
-    if (p) { dev_free(p, pooled, fs); if (t) t->sub(bytes); }
+    if (p) { if (!carved) dev_free(p, pooled, fs); if (t) t->sub(bytes); }
     p = nullptr;
     bytes = 0;
-    pooled = false;
+    pooled = carved = false;
   }
   cudaError_t alloc(size_t b, Tracker *tr) {
     release();
     bytes = b ? b : 16;
     t = tr;
+    Arena *ar = thread_pool().arena;
+    if (ar && ar->fits(bytes)) {
+      p = ar->take(bytes);
+      carved = true;
+      if (t) t->add(bytes);
+      return cudaSuccess;
+    }
     pooled = thread_pool().pool != nullptr;
     cudaError_t e = dev_alloc(&p, bytes, &fs);
     if (e != cudaSuccess) { p = nullptr; bytes = 0; pooled = false; return e; }
@@ -137,6 +175,7 @@ struct rak_graph {
   float plan_ms = 0, h2d_ms = 0;
   size_t off_cap = 0, tgt_cap = 0, wt_cap = 0;  // bytes allocated for an owned copy
   void *wt_alloc = nullptr;                      // owned weight buffer (wt may be null: unit weights)
+  bool arrays_carved = false;                    // owned arrays lie in the call's arena
   bool arrays_pooled = false;                    // owned arrays come from a server slot's pool
   cudaStream_t arrays_fs = nullptr;              // ... and are freed on this stream
   rak_host_detail::RunBufs bufs;  // run buffers reused across runs
@@ -218,14 +257,61 @@ rak_status from_cuda(rak_ctx *ctx, cudaError_t e, const char *what) {
 
 struct Events {
   cudaEvent_t e[6] = {};
-  Events() { for (auto &x : e) cudaEventCreate(&x); }
-  ~Events() { for (auto &x : e) if (x) cudaEventDestroy(x); }
+  rak_ctx *ctx;
+  explicit Events(rak_ctx *c) : ctx(c) {
+    for (auto &x : e) {
+      if (!ctx->events.empty()) { x = ctx->events.back(); ctx->events.pop_back(); }
+      else cudaEventCreate(&x);
+    }
+  }
+  Events(const Events &) = delete;
+  Events &operator=(const Events &) = delete;
+  ~Events() { for (auto &x : e) if (x) ctx->events.push_back(x); }
   float ms(int a, int b) const {
     float t = 0;
     cudaEventElapsedTime(&t, e[a], e[b]);
     return t;
   }
 };
+
+// This thread's buffers come from one block of `bytes` until the scope ends: the context's kept scratch, or a
+// block of the call's own that is freed with the scope. Where there is no room for the block in one piece, the
+// buffers are allocated one by one as without a scope.
+struct ArenaScope {
+  rak_host_detail::PoolTarget saved;
+  rak_host_detail::Arena arena;
+  void *own = nullptr;
+  ArenaScope(rak_ctx *ctx, size_t bytes, bool keep) : saved(rak_host_detail::thread_pool()) {
+    if (saved.pool || saved.arena) return;   // a pool serves already
+    if (keep && bytes <= rak_ctx::SCRATCH_KEEP) {
+      bytes = std::max(bytes, size_t(1) << 20);
+      if (ctx->scratch_bytes < bytes) {
+        if (ctx->scratch) cudaFree(ctx->scratch);
+        ctx->scratch = nullptr;
+        ctx->scratch_bytes = 0;
+        if (cudaMalloc(&ctx->scratch, bytes) == cudaSuccess) ctx->scratch_bytes = bytes;
+        else { ctx->scratch = nullptr; cudaGetLastError(); }
+      }
+      arena.base = static_cast<char *>(ctx->scratch);
+      arena.size = ctx->scratch_bytes;
+    } else {
+      if (cudaMalloc(&own, bytes) == cudaSuccess) { arena.base = static_cast<char *>(own); arena.size = bytes; }
+      else { own = nullptr; cudaGetLastError(); }
+    }
+    if (arena.base) rak_host_detail::thread_pool().arena = &arena;
+  }
+  ArenaScope(const ArenaScope &) = delete;
+  ArenaScope &operator=(const ArenaScope &) = delete;
+  ~ArenaScope() {
+    rak_host_detail::thread_pool() = saved;
+    if (own) cudaFree(own);
+  }
+};
+size_t arena_of(std::initializer_list<size_t> buffers) {
+  size_t b = 0;
+  for (size_t x : buffers) b += rak_host_detail::Arena::rounded(x);
+  return b;
+}
 
 struct Resolved {
   int slots, mode, rescan, pickless, check_on_pickless, iters, start, validate, modularity, repeat, rule, order;
@@ -404,7 +490,7 @@ rak_status build_plan(rak_ctx *ctx, rak_graph *gr, const Layout &ly, Tracker *tr
   gr->ly = ly;
   const int64_t n = gr->n;
   const int nk = nkeys_of(ly);
-  Events ev;
+  Events ev(ctx);
   cudaEventRecord(ev.e[0], st);
   const size_t n4 = size_t(std::max<int64_t>(n, 1)) * 4;
   RAK_TRY(ctx, ensure(gr->p_order, n4));
@@ -489,13 +575,22 @@ rak_status graph_create(rak_ctx *ctx, const rak_csr *g, const Resolved &r, Track
     // a host graph is checked on the device once uploaded (below): the copies touch only the
     // n + 1 offsets and m edges it declares, and the device reads it ~100x faster than the host
     gr->owns = true;
-    Events ev;
+    Events ev(ctx);
     void *po = nullptr, *pt = nullptr, *pw = nullptr;
     gr->arrays_pooled = rak_host_detail::thread_pool().pool != nullptr;
-    cudaError_t e = rak_host_detail::dev_alloc(&po, ob, &gr->arrays_fs);
-    if (e == cudaSuccess) e = rak_host_detail::dev_alloc(&pt, size_t(std::max<int64_t>(g->m, 1)) * 4, &gr->arrays_fs);
-    if (e == cudaSuccess && g->weights)
-      e = rak_host_detail::dev_alloc(&pw, size_t(std::max<int64_t>(g->m, 1)) * 4, &gr->arrays_fs);
+    const size_t eb = size_t(std::max<int64_t>(g->m, 1)) * 4;
+    rak_host_detail::Arena *ar = rak_host_detail::thread_pool().arena;
+    cudaError_t e = cudaSuccess;
+    if (ar && ar->fits(arena_of({ob, eb, g->weights ? eb : 0}))) {
+      gr->arrays_carved = true;
+      po = ar->take(ob);
+      pt = ar->take(eb);
+      if (g->weights) pw = ar->take(eb);
+    } else {
+      e = rak_host_detail::dev_alloc(&po, ob, &gr->arrays_fs);
+      if (e == cudaSuccess) e = rak_host_detail::dev_alloc(&pt, eb, &gr->arrays_fs);
+      if (e == cudaSuccess && g->weights) e = rak_host_detail::dev_alloc(&pw, eb, &gr->arrays_fs);
+    }
     gr->off = po; gr->tgt = static_cast<uint32_t *>(pt); gr->wt = static_cast<float *>(pw);
     gr->off_cap = ob;
     gr->tgt_cap = size_t(std::max<int64_t>(g->m, 1)) * 4;
@@ -514,6 +609,7 @@ rak_status graph_create(rak_ctx *ctx, const rak_csr *g, const Resolved &r, Track
     gr->h2d_ms = ev.ms(0, 1);
   }
   if (r.validate) {
+    ArenaScope scope(ctx, arena_of({4}), true);
     DevBuf bad;
     cudaError_t e = bad.alloc(4, tr);
     unsigned int hbad = 0;
@@ -536,7 +632,7 @@ rak_status ensure_renumbered(rak_ctx *ctx, rak_graph *gr, Tracker *tr) {
   cudaStream_t st = ctx->stream;
   const int64_t n = gr->n, m = gr->m;
   const size_t ob = gr->off64 ? 8 : 4;
-  Events ev;
+  Events ev(ctx);
   cudaEventRecord(ev.e[0], st);
   RAK_TRY(ctx, ensure(gr->rn_inv, size_t(n) * 4));
   RAK_TRY(ctx, ensure(gr->rn_ident, size_t(n) * 4));
@@ -585,8 +681,9 @@ rak_status run_resident(rak_ctx *ctx, rak_graph *gr, const uint32_t *q, const ui
   RAK_TRY(ctx, ensure(b.moved, nh * 4));
   RAK_TRY(ctx, ensure(b.skk, nc * size_t(r.slots) * 4));
   RAK_TRY(ctx, ensure(b.skw, nc * size_t(r.slots) * 4));
-  RAK_TRY(ctx, ensure(b.stats, size_t(iters) * rak::STATS_STRIDE * 8));
-  RAK_TRY(ctx, ensure(b.rs, rak::RUN_STATE_BYTES));
+  // the launch's state behind its counters: cleared by one memset, read back by one copy
+  const size_t stat_bytes = size_t(iters) * rak::STATS_STRIDE * 8, tally_bytes = stat_bytes + rak::RUN_STATE_BYTES;
+  RAK_TRY(ctx, ensure(b.stats, tally_bytes));
   // asynchronous id-label runs work on the graph renumbered in work order (rak_renumber.cu)
   // by default only resident graphs, run again and again, pay for the copy (R-MAT scale 27: about
   // 80 ms once, 26 ms less per run), and only large dense ones: on a sparse R-MAT (scale 25, average
@@ -616,7 +713,7 @@ rak_status run_resident(rak_ctx *ctx, rak_graph *gr, const uint32_t *q, const ui
   a.vcom0 = vcom0; a.vcom1 = b.vcom1.as<uint32_t>(); a.aff0 = b.aff0.as<uint8_t>(); a.aff1 = b.aff1.as<uint8_t>();
   a.hub_arrive = b.arrive.as<uint32_t>(); a.hub_claim = b.claim.as<uint32_t>(); a.hub_moved = b.moved.as<int32_t>();
   a.sk_keys = b.skk.as<uint32_t>(); a.sk_wts = b.skw.as<float>();
-  a.stats = b.stats.as<unsigned long long>(); a.rs = b.rs.p;
+  a.stats = b.stats.as<unsigned long long>(); a.rs = b.stats.as<unsigned char>() + stat_bytes;
   a.iters = r.iters; a.start_iter = r.start; a.tolerance = r.tol; a.pickless_step = r.pickless;
   a.check_on_pickless = r.check_on_pickless; a.rescan = r.rescan; a.mark_test = rak::mark_test_for(a.n, gr->m); a.gpu_rule = r.rule == 2; a.alt = rak::alt_for(r.slots, r.mode, a.gpu_rule, false, n, gr->m, gr->ly, gr->rg); a.timeout_ns = r.timeout_ns; a.tie_until = r.tie_until; a.stage = r.stage; a.grid_cap = r.max_blocks;
   a.dense_moved_edges = rak::dense_threshold(r.mode, r.dense_pct, gr->m);
@@ -644,16 +741,18 @@ rak_status run_resident(rak_ctx *ctx, rak_graph *gr, const uint32_t *q, const ui
     gr->ref_ready = true;
   }
   if (ref_labels && tr) tr->add(gr->ref_ks.bytes + gr->ref_pos.bytes);
-  Events ev;
+  Events ev(ctx);
   float t_init = 0, t_mark = 0, t_all = 0, t_loop = 0;
   rak::RunStateHost hs{};
-  std::vector<unsigned long long> stats(size_t(iters) * rak::STATS_STRIDE, 0);
+  std::vector<unsigned long long> tally(tally_bytes / 8);
+  const unsigned long long *stats = tally.data();
   for (int rep = 0; rep < r.repeat; ++rep) {
-    RAK_TRY(ctx, cudaMemsetAsync(b.arrive.p, 0, b.arrive.bytes, st));
-    RAK_TRY(ctx, cudaMemsetAsync(b.claim.p, 0, b.claim.bytes, st));
-    RAK_TRY(ctx, cudaMemsetAsync(b.moved.p, 0xFF, b.moved.bytes, st));
-    RAK_TRY(ctx, cudaMemsetAsync(b.stats.p, 0, b.stats.bytes, st));
-    RAK_TRY(ctx, cudaMemsetAsync(b.rs.p, 0, b.rs.bytes, st));
+    if (gr->nhub > 0) {
+      RAK_TRY(ctx, cudaMemsetAsync(b.arrive.p, 0, nh * 4, st));
+      RAK_TRY(ctx, cudaMemsetAsync(b.claim.p, 0, nh * 4, st));
+      RAK_TRY(ctx, cudaMemsetAsync(b.moved.p, 0xFF, nh * 4, st));
+    }
+    RAK_TRY(ctx, cudaMemsetAsync(b.stats.p, 0, tally_bytes, st));
     cudaEventRecord(ev.e[0], st);
     if (renum) {
       RAK_TRY(ctx, rak::launch_renumbered_init(gr->order, q, ref_labels ? gr->ref_pos.as<uint32_t>() : nullptr, flags,
@@ -667,21 +766,20 @@ rak_status run_resident(rak_ctx *ctx, rak_graph *gr, const uint32_t *q, const ui
     cudaEventRecord(ev.e[1], st);
     if (!renum) RAK_TRY(ctx, rak::launch_init_flags(a.aff0, sync ? a.aff1 : nullptr, flags, n, st));
     cudaEventRecord(ev.e[2], st);
-    if (a.pull) RAK_TRY(ctx, rak::launch_symmetry(a.off, gr->off64, a.tgt, n, gr->m, nullptr, nullptr, b.rs.p, st));
+    if (a.pull) RAK_TRY(ctx, rak::launch_symmetry(a.off, gr->off64, a.tgt, n, gr->m, nullptr, nullptr, a.rs, st));
     if (r.iters > 0) {
       int grid = 0;
       RAK_TRY(ctx, rak::launch_lpa(a, r.slots, r.mode, gr->off64, st, &grid));
     }
     cudaEventRecord(ev.e[3], st);
+    if (rep + 1 == r.repeat) RAK_TRY(ctx, cudaMemcpyAsync(tally.data(), b.stats.p, tally_bytes, cudaMemcpyDeviceToHost, st));
     RAK_TRY(ctx, cudaStreamSynchronize(st));
     t_init += ev.ms(0, 1);
     t_mark += ev.ms(1, 2);
     t_loop += ev.ms(2, 3);
     t_all += ev.ms(0, 3);
   }
-  RAK_TRY(ctx, cudaMemcpyAsync(&hs, b.rs.p, sizeof(hs), cudaMemcpyDeviceToHost, st));
-  RAK_TRY(ctx, cudaMemcpyAsync(stats.data(), b.stats.p, stats.size() * 8, cudaMemcpyDeviceToHost, st));
-  RAK_TRY(ctx, cudaStreamSynchronize(st));
+  std::memcpy(&hs, tally.data() + stat_bytes / 8, sizeof(hs));
   if (hs.error) {
     set_err(ctx, "device-side wait gave up (status %u)", hs.error);
     return rak_status(hs.error);
@@ -690,7 +788,7 @@ rak_status run_resident(rak_ctx *ctx, rak_graph *gr, const uint32_t *q, const ui
   if (sync && (done & 1)) RAK_TRY(ctx, cudaMemcpyAsync(a.vcom0, a.vcom1, size_t(n) * 4, cudaMemcpyDeviceToDevice, st));
   if (renum) RAK_TRY(ctx, rak::launch_renumbered_gather(b.lab.as<uint32_t>(), gr->rn_inv.as<uint32_t>(), n, vcom0, st));
   if (ref_labels) RAK_TRY(ctx, rak::launch_labels_to_ids(vcom0, gr->ref_ks.as<uint32_t>(), n, st));
-  RAK_TRY(ctx, cudaStreamSynchronize(st));
+  if ((sync && (done & 1)) || renum || ref_labels) RAK_TRY(ctx, cudaStreamSynchronize(st));
   if (res) {
     res->iterations = done;
     res->time_ms = t_all / float(r.repeat);
@@ -700,7 +798,7 @@ rak_status run_resident(rak_ctx *ctx, rak_graph *gr, const uint32_t *q, const ui
     res->traversed_edges = res->processed_vertices = res->moved_vertices = res->moved_edges = res->marked_edges = 0;
     res->dense_iterations = 0;
     for (int i = 0; i < done; ++i) {
-      const unsigned long long *st_i = &stats[size_t(i) * rak::STATS_STRIDE];
+      const unsigned long long *st_i = stats + size_t(i) * rak::STATS_STRIDE;
       res->traversed_edges += st_i[rak::STAT_EDGES];
       res->processed_vertices += st_i[rak::STAT_PROCESSED];
       res->moved_vertices += st_i[rak::STAT_CHANGED];
@@ -716,8 +814,11 @@ rak_status run_resident(rak_ctx *ctx, rak_graph *gr, const uint32_t *q, const ui
   return RAK_OK;
 }
 
+size_t modularity_arena(int64_t n) { return arena_of({4, size_t(std::max<int64_t>(n, 1)) * 8, 4 * 8}); }
+
 rak_status modularity_dev(rak_ctx *ctx, const void *off, bool off64, const uint32_t *tgt, const float *wt, int64_t n, int64_t m,
                           const uint32_t *labels, Tracker *tr, double *q) {
+  ArenaScope scope(ctx, modularity_arena(n), true);
   DevBuf ctot, sums;
   RAK_TRY(ctx, ctot.alloc(size_t(std::max<int64_t>(n, 1)) * 8, tr));
   RAK_TRY(ctx, sums.alloc(4 * 8, tr));
@@ -730,6 +831,30 @@ rak_status modularity_dev(rak_ctx *ctx, const void *off, bool off64, const uint3
   if (h[3] > 0) { set_err(ctx, "membership holds labels >= n"); return RAK_ERR_INVALID_ARGUMENT; }
   *q = h[1] > 0 ? h[0] / h[1] - h[2] / (h[1] * h[1]) : 0.0;
   return RAK_OK;
+}
+
+// What a one-shot run holds beside a device-located graph: the uploaded graph and labels (host graphs), the
+// plan with its sort space, the run's buffers and, where asked for, the reference order and the modularity's
+// sums. Split vertices are counted at most.
+size_t one_shot_arena(const rak_csr *g, const uint32_t *q, const rak_options *o, const Resolved &r) {
+  const size_t n = size_t(std::max<int64_t>(g->n, 1)), m = size_t(std::max<int64_t>(g->m, 1));
+  const size_t hubs = m / size_t(r.ly.hub_min + 1) + 1, chunks = m / size_t(r.ly.hub_chunk) + hubs;
+  size_t sort = 0;
+  if (g->n > 0) rak::plan_sort(nullptr, nullptr, nullptr, nullptr, g->n, 11, nullptr, &sort, nullptr);
+  size_t b = arena_of({4, n * 4, n * 4, n * 4, n * 4, size_t(nkeys_of(r.ly)) * 8, sort, hubs * 8, (hubs + 1) * 8, chunks * 4,
+                       n + 16, hubs * 4, hubs * 4, hubs * 4, chunks * size_t(r.slots) * 4, chunks * size_t(r.slots) * 4,
+                       size_t(std::max(r.iters, 1)) * rak::STATS_STRIDE * 8 + rak::RUN_STATE_BYTES});
+  if (r.mode != RAK_MODE_ASYNC) b += arena_of({n * 4 + 16, n + 16});
+  if (r.order == 2) b += arena_of({n * 4, n * 4, rak::ref_order_scratch_bytes(g->n, 1)});
+  if (r.modularity) b += arena_of({4, n * 8, 4 * 8});
+  if (g->location == RAK_HOST) {
+    const size_t ob = (n + 1) * (g->offset_bits == 64 ? 8 : 4);
+    b += arena_of({ob, m * 4, n * 4 + 16});
+    if (g->weights) b += arena_of({m * 4});
+    if (q) b += arena_of({n * 4 + 16});
+    if (o && o->initial_flags) b += arena_of({n + 16});
+  }
+  return b;
 }
 
 }  // namespace
@@ -843,7 +968,7 @@ rak_status rak_graph_create(rak_ctx *ctx, const rak_csr *g, const rak_options *o
 rak_status rak_graph_destroy(rak_graph *gr) {
   if (!gr) return RAK_ERR_INVALID_ARGUMENT;
   cudaSetDevice(gr->device);
-  if (gr->owns) {
+  if (gr->owns && !gr->arrays_carved) {
     rak_host_detail::dev_free(const_cast<void *>(gr->off), gr->arrays_pooled, gr->arrays_fs);
     rak_host_detail::dev_free(const_cast<uint32_t *>(gr->tgt), gr->arrays_pooled, gr->arrays_fs);
     rak_host_detail::dev_free(gr->wt_alloc, gr->arrays_pooled, gr->arrays_fs);
@@ -891,6 +1016,8 @@ rak_status rak_lowmem_cuda(rak_ctx *ctx, const rak_csr *g, const uint32_t *q, co
   // with a context pool, this call's buffers are stream-ordered allocations from it (kept mapped
   // between calls up to the pool's threshold); otherwise cudaMalloc/cudaFree
   rak_host_detail::PoolScope scope(ctx->keep > 0 ? ctx->pool : nullptr, ctx->stream);
+  RAK_CHECK(check_csr_shape(ctx, g));
+  ArenaScope arena(ctx, one_shot_arena(g, q, o, r), false);   // given back when the call ends
   Tracker tr;
   rak_graph *gr = nullptr;
   RAK_CHECK(graph_create(ctx, g, r, &tr, &gr));
@@ -906,7 +1033,7 @@ rak_status rak_lowmem_cuda(rak_ctx *ctx, const rak_csr *g, const uint32_t *q, co
   }
   DevBuf labels, qd, fd;
   RAK_TRY(ctx, labels.alloc(size_t(n) * 4 + 16, &tr));
-  Events ev;
+  Events ev(ctx);
   cudaEventRecord(ev.e[0], ctx->stream);
   if (q) {
     RAK_TRY(ctx, qd.alloc(size_t(n) * 4 + 16, &tr));
@@ -943,8 +1070,10 @@ rak_status rak_graph_step(rak_ctx *ctx, rak_graph *gr, const rak_options *o, int
   cudaStream_t st = ctx->stream;
   const int64_t n = gr->n;
   const bool sync = r.mode != RAK_MODE_ASYNC;
-  RunBufs b;
   const size_t nh = size_t(std::max<int64_t>(gr->nhub, 1)), nc = size_t(std::max<int64_t>(gr->nchunks, 1));
+  ArenaScope scope(ctx, arena_of({nh * 4, nh * 4, nh * 4, nc * size_t(r.slots) * 4, nc * size_t(r.slots) * 4,
+                                  rak::STATS_STRIDE * 8, rak::RUN_STATE_BYTES}), true);
+  RunBufs b;
   RAK_TRY(ctx, b.arrive.alloc(nh * 4, nullptr));
   RAK_TRY(ctx, b.claim.alloc(nh * 4, nullptr));
   RAK_TRY(ctx, b.moved.alloc(nh * 4, nullptr));
@@ -993,6 +1122,7 @@ rak_status rak_modularity_f64(rak_ctx *ctx, const rak_csr *g, const uint32_t *me
   RAK_CHECK(check_csr_shape(ctx, g));
   RAK_TRY(ctx, cudaSetDevice(ctx->device));
   if (g->location == RAK_DEVICE) {
+    ArenaScope scope(ctx, modularity_arena(g->n), true);
     DevBuf bad;
     unsigned int hbad = 0;
     RAK_TRY(ctx, bad.alloc(4, nullptr));
@@ -1254,9 +1384,11 @@ rak_status batch_enqueue(rak_ctx *ctx, rak_batch *b, const uint32_t *q, const Re
   const int64_t n = gr->n, G = b->ngraphs;
   const bool sync = r.mode != RAK_MODE_ASYNC;
   const int iters = std::max(r.iters, 1);
-  RAK_TRY(ctx, cudaMemsetAsync(rb.arrive.p, 0, rb.arrive.bytes, st));
-  RAK_TRY(ctx, cudaMemsetAsync(rb.claim.p, 0, rb.claim.bytes, st));
-  RAK_TRY(ctx, cudaMemsetAsync(rb.moved.p, 0xFF, rb.moved.bytes, st));
+  if (gr->nhub > 0) {
+    RAK_TRY(ctx, cudaMemsetAsync(rb.arrive.p, 0, rb.arrive.bytes, st));
+    RAK_TRY(ctx, cudaMemsetAsync(rb.claim.p, 0, rb.claim.bytes, st));
+    RAK_TRY(ctx, cudaMemsetAsync(rb.moved.p, 0xFF, rb.moved.bytes, st));
+  }
   RAK_TRY(ctx, cudaMemsetAsync(rb.stats.p, 0, size_t(iters) * rak::STATS_STRIDE * 8, st));
   RAK_TRY(ctx, cudaMemsetAsync(rb.rs.p, 0, rak::RUN_STATE_BYTES, st));
   RAK_TRY(ctx, cudaMemsetAsync(b->gdone.p, 0, size_t(G) + 16, st));
@@ -1867,7 +1999,8 @@ rak_status rak_server_create(rak_ctx *ctx, const rak_server_options *o, rak_serv
   rak_status st = resolve(ctx, &o->run, &s->run);
   batch_default_order(&o->run, &s->run);
   if (st != RAK_OK) { delete s; return st; }
-  s->grid_cap = std::max(1, ctx->sms * 3 / o->slots);
+  // a slot's share of the blocks that fit: four per SM (asynchronous launches keep the three their pace was set with)
+  s->grid_cap = std::max(1, ctx->sms * (s->run.mode == RAK_MODE_ASYNC ? 3 : 4) / o->slots);
   for (int i = 0; i < o->slots; ++i) {
     s->slots.push_back(std::make_unique<ServerSlot>());
     ServerSlot &sl = *s->slots.back();
