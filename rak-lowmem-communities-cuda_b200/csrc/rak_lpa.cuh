@@ -632,24 +632,25 @@ __device__ __forceinline__ void exact_group_scan(Sketch<S> &sk, uint32_t u, int6
   }
 }
 
-// The same sequential scan of one vertex by a whole warp, 32 edges at a time, for long lists. Every lane holds
-// the keys and, slot by slot, which of the 32 edges hit them (a vote each). Edges up to the first miss are
-// applied at once by slot i's lane, which holds its weight: unit weights by counting, others by adding its
-// edges' weights in order. Then the miss is settled (insert or decrement); the edges that hit an inserted key
-// are known from one label match at the start (weights in every lane, without votes: slower, 15.9 against 11.9 ms). With rescan a second
-// pass does the same with the final keys. exact_group_scan instead takes every edge through every lane's copy
-// of the sketch, about 430 cycles an edge for both passes, and the longest list is the iteration. Measured on
-// B200, exact synchronous runs, before -> now: R-MAT scale 16 ef 16 22.8 -> 10.5 ms, weighted (marking instead of
-// pulling before) 55 -> 35 ms, scale 18 (the same) 147 -> 82 ms.
+// The same sequential scan of one vertex by a whole warp, 32 edges at a time, for long lists. Lane i < S holds
+// slot i: its key, its weight and which of the 32 edges hit it (a vote per slot). Edges up to the first miss are
+// applied at once, each slot's by its lane: unit weights by counting, others by adding in order. Then the misses
+// that follow each other without a hit: with free slots, as many as there are take them together, the first the
+// last free one and so on, if their labels differ (a label that repeats would hit what the first one inserted;
+// one match at the start tells) and their weights are not zero; with none, unit weights drop by as many misses as
+// the smallest weight bears. With rescan a second pass does the same with the final keys. exact_group_scan
+// instead takes every edge through every lane's copy of the sketch, about 430 cycles an edge for both passes, and
+// the longest list is the iteration. Measured on B200, exact synchronous runs, before -> misses one at a time ->
+// this: R-MAT scale 16 ef 16 22.8 -> 10.5 -> 5.8 ms, weighted 55 -> 35 -> 22 ms, scale 18 147 -> 82 -> 36 ms (the
+// last two with marking instead of pulling before).
 template <int S, bool UNIT>
 __device__ __forceinline__ void exact_warp_scan(Sketch<S> &sk, uint32_t u, int64_t eb, int64_t ee, bool rescan,
                                                 const uint32_t *tgt, const float *wt, const uint32_t *vin,
                                                 uint32_t base) {
   const int lane = threadIdx.x & 31;
-  uint32_t k[S], num = 0u, low = 0u;   // unit weights: slot `lane` weighs num - low
+  const unsigned before = (1u << lane) - 1u;   // the lanes before this one
+  uint32_t k = NONE, num = 0u, low = 0u;       // slot `lane`; unit weights: it weighs num - low
   float w = 0.0f;
-#pragma unroll
-  for (int i = 0; i < S; ++i) k[i] = NONE;
   for (int pass = 0; pass < (rescan ? 2 : 1); ++pass) {
     if (pass == 1) { num = low = 0u; w = 0.0f; }
     uint32_t t = eb + lane < ee ? base + ld_edge(tgt + eb + lane) : u;
@@ -663,17 +664,21 @@ __device__ __forceinline__ void exact_warp_scan(Sketch<S> &sk, uint32_t u, int64
       const uint32_t c2 = t2 != u ? ld_label(vin + t2) : NONE;
       const bool ok = t != u;   // self-loops and positions past the end take no part
       const unsigned valid = __ballot_sync(FULL, ok);
-      unsigned m[S], hits = 0u, own = 0u;   // edges that hit slot i; any slot; slot `lane`
+      unsigned own = 0u, hits = 0u;   // edges that hit slot `lane`; any slot
 #pragma unroll
       for (int i = 0; i < S; ++i) {
-        m[i] = __ballot_sync(FULL, ok && c == k[i]);
-        hits |= m[i];
-        if (lane == i) own = m[i];
+        const uint32_t ki = __shfl_sync(FULL, k, i);
+        const unsigned m = __ballot_sync(FULL, ok && c == ki);
+        hits |= m;
+        if (lane == i) own = m;
       }
       unsigned left = FULL;   // edges not applied yet
       unsigned miss = pass == 0 ? valid & ~hits : 0u;
-      unsigned peers = 0u;
-      if (miss) peers = __match_any_sync(FULL, c);
+      unsigned peers = 0u, light = 0u;   // edges of the same label; edges of weight 0
+      if (miss) {
+        peers = __match_any_sync(FULL, c) & valid;
+        if constexpr (!UNIT) light = __ballot_sync(FULL, x == 0.0f);
+      }
       for (;;) {
         const unsigned now = left & (miss ? (miss & (0u - miss)) - 1u : FULL);
         if constexpr (UNIT) {
@@ -689,25 +694,38 @@ __device__ __forceinline__ void exact_warp_scan(Sketch<S> &sk, uint32_t u, int64
         }
         if (!miss) break;
         const int p = __ffs(int(miss)) - 1;
-        left = ~((2u << p) - 1u);
-        const uint32_t cp = __shfl_sync(FULL, c, p);
-        const unsigned next = __shfl_sync(FULL, peers, p) & valid;
-        const float xp = UNIT ? 1.0f : __shfl_sync(FULL, x, p);
         const unsigned open = __ballot_sync(FULL, lane < S && (UNIT ? num == low : w == 0.0f));
+        int done = 1;   // misses settled now: edges p .. p + done - 1
         if (open) {
-          const int f = 31 - __clz(int(open));   // the last free slot
-#pragma unroll
-          for (int i = 0; i < S; ++i)
-            if (i == f) { k[i] = cp; m[i] = next; }
-          if (lane == f) { own = next; num = low + 1u; w = xp; }
+          // misses from p on whose label has not come up since p
+          const unsigned again = __ballot_sync(FULL, ((peers & before) >> p) != 0u);
+          const unsigned run = (miss & ~again) >> p;
+          const int len = run == FULL ? 32 : __ffs(int(~run)) - 1, room = __popc(open);
+          done = len < room ? len : room;
+          if (!UNIT && ((light >> p) & ((done == 32 ? 0u : 1u << done) - 1u)) != 0u) done = 1;
+          const int j = __popc(open & ~before & ~(1u << lane));   // free slots after this one
+          const int from = p + (j < done ? j : 0);
+          const uint32_t cn = __shfl_sync(FULL, c, from);
+          const unsigned next = __shfl_sync(FULL, peers, from);
+          const float xn = UNIT ? 1.0f : __shfl_sync(FULL, x, from);
+          if (((open >> lane) & 1u) && j < done) {
+            k = cn;
+            num = low + 1u;
+            w = xn;
+            own = next & ~((2u << from) - 1u);
+          }
+          hits = __reduce_or_sync(FULL, own);
         } else if constexpr (UNIT) {
-          low += 1u;
+          const unsigned run = miss >> p;
+          const unsigned len = run == FULL ? 32u : unsigned(__ffs(int(~run)) - 1);
+          const unsigned bears = __reduce_min_sync(FULL, lane < S ? num - low : 32u);
+          done = int(len < bears ? len : bears);
+          low += unsigned(done);
         } else {
+          const float xp = __shfl_sync(FULL, x, p);
           w = fmaxf(__fsub_rn(w, xp), 0.0f);
         }
-        hits = 0u;
-#pragma unroll
-        for (int i = 0; i < S; ++i) hits |= m[i];
+        left = p + done > 31 ? 0u : FULL << (p + done);
         miss = valid & ~hits & left;
       }
       t = t2; x = x2; c = c2;
@@ -715,7 +733,7 @@ __device__ __forceinline__ void exact_warp_scan(Sketch<S> &sk, uint32_t u, int64
   }
 #pragma unroll
   for (int i = 0; i < S; ++i) {
-    sk.k[i] = k[i];
+    sk.k[i] = __shfl_sync(FULL, k, i);
     sk.w[i] = __shfl_sync(FULL, UNIT ? float(num - low) : w, i);
   }
 }
@@ -974,8 +992,8 @@ __device__ __forceinline__ void group_item(const LpaArgs &a, const Regions &rg, 
   Sketch<S> sk;
   sk_clear<S, RULE>(sk, v.d);
   if constexpr (MODE == MODE_SYNC) {
-    // groups of 8 lanes or more (1024 edges or more): their lists one after the other by the whole warp, still
-    // the shorter way (32 lists' worth of batches against one list edge by edge); smaller groups side by side
+    // groups of 8 lanes or more (1024 edges or more): their lists one after the other by the whole warp; smaller
+    // groups side by side (lists one after the other from 2 lanes on: R-MAT scale 12 without rescan 2.0 -> 3.5 ms)
     if (S > 1 && G >= 8) {
       for (int o = 0; o < 32; o += G) {
         if (__shfl_sync(FULL, int(v.active), o) == 0) continue;
