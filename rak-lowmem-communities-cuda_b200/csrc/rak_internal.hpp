@@ -201,9 +201,10 @@ inline int default_label_order(int mode, int slots) { return mode == MODE_ASYNC 
 
 // Per-iteration counters written by the LPA kernel.
 // STAT_PHASE: how the iteration treated the frontier (bit 0: its moves marked no neighbours; bit 1:
-// it processed every vertex), written by the asynchronous single-graph kernel.
+// it processed every vertex), written by the asynchronous single-graph kernel. STAT_IDLE: the same word in the
+// synchronous modes, from bit 1 on the longest list of region 1 that was not in the active set.
 enum Stat { STAT_CHANGED = 0, STAT_EDGES = 1, STAT_PROCESSED = 2, STAT_HUBS_MOVED = 3, STAT_MOVED_EDGES = 4, STAT_WORK = 5,
-            STAT_PHASE = 6, STAT_WIDE = 7 };
+            STAT_PHASE = 6, STAT_IDLE = 6, STAT_WIDE = 7 };
 constexpr int STATS_STRIDE = 8;
 
 // Persistent cooperative launch of all iterations; grid chosen from occupancy. `batch` selects the

@@ -826,22 +826,34 @@ __device__ __forceinline__ bool lane_pull(uint32_t u, int64_t e, int64_t ee, con
 }
 
 // The same by the aligned groups of G lanes, each for its own vertex (want: the group looks at all);
-// every lane of the warp calls it, and a group's lanes get the same answer.
+// every lane of the warp calls it, and a group's lanes get the same answer. One edge a lane first, which
+// mostly finds one; then PULL_BATCH at a time: a list without a moved neighbour is read to its end, and with
+// one edge in flight a lane 60000 edges took a warp 0.7 ms.
+constexpr int PULL_BATCH = 8;
 __device__ __forceinline__ bool group_pull(bool want, uint32_t u, int64_t eb, int64_t ee, int s, int G, int grp,
                                            const uint32_t *tgt, const uint8_t *fin, uint32_t base) {
   const unsigned gm = G == 32 ? FULL : ((1u << G) - 1u) << (grp * G);
-  bool found = false;
-  for (int64_t e = eb + s;; e += G) {
-    const bool more = want && !found && e < ee;
-    bool hit = false;
-    if (more) {
-      const uint32_t t = base + ld_edge(tgt + e);
-      hit = t != u && fin[t] != 0;
-    }
-    const unsigned hits = __ballot_sync(FULL, hit);
-    found = found || (hits & gm) != 0;
-    if (__ballot_sync(FULL, more && !found) == 0) return found;
+  int64_t e = eb + s;
+  uint32_t any = 0u;
+  if (want && e < ee) {
+    const uint32_t t = base + ld_edge(tgt + e);
+    any = t != u ? uint32_t(fin[t]) : 0u;
   }
+  bool found = (__ballot_sync(FULL, any != 0u) & gm) != 0;
+  e += G;
+  while (__ballot_sync(FULL, want && !found && e < ee)) {
+    if (want && !found && e < ee) {
+      uint32_t t[PULL_BATCH];
+#pragma unroll
+      for (int j = 0; j < PULL_BATCH; ++j) t[j] = e + j * G < ee ? base + ld_edge(tgt + e + j * G) : u;
+#pragma unroll
+      for (int j = 0; j < PULL_BATCH; ++j) any |= t[j] != u ? uint32_t(fin[t[j]]) : 0u;
+    }
+    const unsigned hits = __ballot_sync(FULL, any != 0u);   // by every lane, outside any condition
+    found = found || (hits & gm) != 0;
+    e += int64_t(PULL_BATCH) * G;
+  }
+  return found;
 }
 
 // ---- work items: open (what to scan), close (choose, move) --------------------------------------
@@ -937,22 +949,36 @@ struct GroupVertex {
   int64_t eb, ee;
   bool valid, active;
 };
-template <class O, bool BATCH>
+
+// The longest list of region 1 that an iteration left out of its active set (STAT_IDLE), for pulls_next: the
+// lane that calls it speaks for its vertex u.
+template <class O>
+__device__ __forceinline__ void note_idle(const LpaArgs &a, const G_<O> &g, uint32_t u, int it) {
+  const unsigned long long deg = (unsigned long long)(__ldg(g.off + u + 1) - __ldg(g.off + u));
+  atomicMax(a.stats + STATS_STRIDE * it + STAT_IDLE, deg << 1);   // bit 0 is STAT_PHASE's
+}
+
+template <int MODE, class O, bool BATCH>
 __device__ __forceinline__ GroupVertex group_open(const LpaArgs &a, const Regions &rg, const G_<O> &g, int r,
-                                                  int64_t local, const uint32_t *vin, const uint8_t *fin, Phase ph) {
+                                                  int64_t local, int it, const uint32_t *vin, const uint8_t *fin,
+                                                  Phase ph) {
   const int G = region_group(r);
   const int lane = threadIdx.x & 31, grp = lane / G, s = lane & (G - 1);
   const int64_t idx = local * (32 / G) + grp;
   GroupVertex v{0, 0, 0, 0, 0, 0, idx < rg.vcount[r], false};
+  bool running = false;
   if (v.valid) {
     v.u = __ldg(a.order + rg.vbegin[r] + idx);
     v.d = vin[v.u];
-    v.active = !graph_of<BATCH>(a, v.u, v.gi, v.base) && (ph.pull_in || ph.all || fin[v.u] != 0);
+    running = !graph_of<BATCH>(a, v.u, v.gi, v.base);
+    v.active = running && (ph.pull_in || ph.all || fin[v.u] != 0);
     if (v.active) { v.eb = int64_t(__ldg(g.off + v.u)); v.ee = int64_t(__ldg(g.off + v.u + 1)); }
   }
   if (ph.pull_in)
     v.active = G == 1 ? v.active && lane_pull(v.u, v.eb, v.ee, g.tgt, fin, v.base)
                       : group_pull(v.active, v.u, v.eb, v.ee, s, G, grp, g.tgt, fin, v.base);
+  if constexpr (MODE != MODE_ASYNC)
+    if (G == 32 && s == 0 && a.pull != 0 && running && !v.active) note_idle(a, g, v.u, it);
   return v;
 }
 // Merges the group's sketches, chooses and moves; true on every lane of the group if it moved.
@@ -988,7 +1014,7 @@ __device__ __forceinline__ void group_item(const LpaArgs &a, const Regions &rg, 
                                            uint8_t *fin, uint8_t *fout, Counters &cnt, StageCtx &sc, Phase ph) {
   const int G = region_group(r);
   const int lane = threadIdx.x & 31, grp = lane / G, s = lane & (G - 1);
-  const GroupVertex v = group_open<O, BATCH>(a, rg, g, r, local, vin, fin, ph);
+  const GroupVertex v = group_open<MODE, O, BATCH>(a, rg, g, r, local, it, vin, fin, ph);
   Sketch<S> sk;
   sk_clear<S, RULE>(sk, v.d);
   if constexpr (MODE == MODE_SYNC) {
@@ -1032,6 +1058,36 @@ struct HubChunk {
   int64_t eb, ee, cb, ce;  // edges of the vertex and of the chunk
   bool active;
 };
+
+// Which split vertices have a neighbour that moved, before iteration `next` pulls: every chunk's warp looks
+// through its own edges, unless a chunk of the vertex has found one, and hub_claim (which only asynchronous
+// launches use otherwise) takes the iteration's number. Each edge is looked at once at most, by as many warps as
+// there are chunks; a search of the whole list by every chunk's warp instead made a settled vertex of a million
+// edges beside moving ones cost 12 ms an iteration (R-MAT graphs, whose first edges find a mover: the same). The
+// caller's barrier comes before and after. A function of its own, not inlined, as wide_items.
+template <class O, bool BATCH>
+__device__ __noinline__ void hub_pull(const LpaArgs &a, const Regions &rg, const uint8_t *movers, int next) {
+  const G_<O> g{static_cast<const O *>(a.off), a.tgt, a.wt};
+  const int lane = threadIdx.x & 31;
+  const int64_t gw = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+  const int64_t nw = (int64_t(gridDim.x) * blockDim.x) >> 5;
+  for (int64_t i = gw; i < a.nchunks; i += nw) {
+    const uint32_t h = __ldg(a.chunk_hub + i);
+    unsigned int known = 0u;
+    if (lane == 0) known = *(volatile unsigned int *)(a.hub_claim + h);
+    if (__shfl_sync(FULL, known, 0) == unsigned(next + 1)) continue;
+    const uint32_t u = __ldg(a.order + rg.vbegin[REG_HUB] + h);
+    uint32_t gi, base;
+    // a batch may be settling its graphs meanwhile: one lane's reading holds for the warp, and either will do
+    if (__shfl_sync(FULL, int(graph_of<BATCH>(a, u, gi, base)), 0)) continue;
+    const int64_t eb = int64_t(__ldg(g.off + u)), ee = int64_t(__ldg(g.off + u + 1));
+    const int64_t cb = eb + (i - __ldg(a.hub_first + h)) * a.hub_chunk;
+    const int64_t ce = cb + a.hub_chunk < ee ? cb + a.hub_chunk : ee;
+    const bool found = group_pull(true, u, cb, ce, lane, 32, 0, g.tgt, movers, base);
+    if (found && lane == 0) *(volatile unsigned int *)(a.hub_claim + h) = unsigned(next + 1);
+  }
+}
+
 template <int MODE, class O, bool BATCH>
 __device__ __forceinline__ HubChunk hub_open(const LpaArgs &a, const Regions &rg, const G_<O> &g, int64_t local, int it,
                                              uint8_t *fin, Phase ph) {
@@ -1050,7 +1106,7 @@ __device__ __forceinline__ HubChunk hub_open(const LpaArgs &a, const Regions &rg
   if (gfin) {
     k.active = false;
   } else if (MODE != MODE_ASYNC) {
-    k.active = ph.pull_in ? group_pull(true, k.u, k.eb, k.ee, lane, 32, 0, g.tgt, fin, k.base) : fin[k.u] != 0;
+    k.active = ph.pull_in ? __ldcg(a.hub_claim + k.h) == unsigned(it + 1) : fin[k.u] != 0;   // hub_pull
   } else {
     // All chunks of u agree on whether u is processed this iteration: the first chunk to get
     // here decides from u's flag (and clears it); the others read the decision.
@@ -1304,7 +1360,7 @@ __device__ __noinline__ Counters wide_items(const LpaArgs &a, const Regions &rg,
         k = hub_open<MODE, O, BATCH>(a, rg, g, local, it, fin, ph);
         ws.u[lane] = k.u; ws.base[lane] = k.base; ws.eb[lane] = k.cb + lane; ws.ee[lane] = k.ce;
       } else {
-        v = group_open<O, BATCH>(a, rg, g, r, local, vin, fin, ph);
+        v = group_open<MODE, O, BATCH>(a, rg, g, r, local, it, vin, fin, ph);
         ws.u[lane] = v.u; ws.base[lane] = v.base; ws.eb[lane] = v.eb + s; ws.ee[lane] = v.ee;
       }
       const unsigned live = __ballot_sync(FULL, r == REG_HUB ? k.active : v.active);
@@ -1350,11 +1406,15 @@ __device__ __noinline__ Counters wide_items(const LpaArgs &a, const Regions &rg,
 
 // Whether iteration it + 1 records its movers for the one after it: when the vertices that moved in
 // iteration it hold a quarter of the edges or more (in the first iteration: when every vertex starts
-// affected). Every block reads the same counter after the barrier, so all agree; the choice changes what
-// the flags hold, not the result.
+// affected), and no list of region 1 that one warp would read to its end in vain is as long as to outlast the
+// iteration: L edges take L / 256 round trips of about half a microsecond, a balanced iteration m / 250 G/s, so
+// L up to m / 512. (Split vertices are searched by all their chunks' warps, hub_pull; the lists of smaller groups
+// are 16 * lane_max edges at most.) Measured on B200, 10 iterations of a settled vertex of 60000 edges beside
+// 60000 vertices that move in pairs: never pulled 0.36 ms, pulled whatever the list 6.95 ms. Every block reads the
+// same counters after the barrier, so all agree; the choice changes what the flags hold, not the result.
 __device__ __forceinline__ bool pulls_next(const LpaArgs &a, int it, bool can_pull) {
-  return can_pull && it + 2 < a.iters &&
-         __ldcg(a.stats + STATS_STRIDE * it + STAT_MOVED_EDGES) * 4ull >= (unsigned long long)a.m;
+  const unsigned long long *st = a.stats + STATS_STRIDE * it, m = (unsigned long long)a.m;
+  return can_pull && it + 2 < a.iters && __ldcg(st + STAT_MOVED_EDGES) * 4ull >= m && (__ldcg(st + STAT_IDLE) >> 1) * 512ull <= m;
 }
 
 // WIDE: the launch has wide items. Launches without any take a kernel that does not hold their code and
@@ -1527,6 +1587,7 @@ __global__ void __launch_bounds__(256, RAK_MIN_BLOCKS) lpa_run(const __grid_cons
       if (lane == 0 && run) atomicAdd(a.running + it, run);
       if constexpr (MODE != MODE_ASYNC) {
         next_out = pulls_next(a, it, can_pull);
+        if (ph.pull_out && a.nchunks > 0) hub_pull<O, BATCH>(a, rg, fout, it + 1);
         uint4 *f4 = reinterpret_cast<uint4 *>(fin);
         const int64_t n16 = a.n >> 4;
         for (int64_t i = tid; i < n16; i += nt) f4[i] = make_uint4(0, 0, 0, 0);
@@ -1546,14 +1607,19 @@ __global__ void __launch_bounds__(256, RAK_MIN_BLOCKS) lpa_run(const __grid_cons
     if constexpr (MODE != MODE_ASYNC) {
       next_out = pulls_next(a, it, can_pull);
       // Every vertex with an edge writes its flag in an iteration that records movers: nothing to clear,
-      // and nothing after the barrier above to wait for unless this one marked split vertices' neighbours.
-      if (next_out && ph.pull_out) continue;
+      // and nothing after the barrier above to wait for unless this one marked split vertices' neighbours or
+      // the next one needs to know which of them have a moved neighbour.
+      const bool clear = !(next_out && ph.pull_out);
+      if (ph.pull_out && a.nchunks > 0) hub_pull<O, BATCH>(a, rg, fout, it + 1);
+      else if (!clear) continue;
       // The flags just read become next iteration's output: clear them.
-      const int64_t tid = int64_t(blockIdx.x) * blockDim.x + threadIdx.x, nt = int64_t(gridDim.x) * blockDim.x;
-      uint4 *f4 = reinterpret_cast<uint4 *>(fin);
-      const int64_t n16 = a.n >> 4;
-      for (int64_t i = tid; i < n16; i += nt) f4[i] = make_uint4(0, 0, 0, 0);
-      for (int64_t i = (n16 << 4) + tid; i < a.n; i += nt) fin[i] = 0;
+      if (clear) {
+        const int64_t tid = int64_t(blockIdx.x) * blockDim.x + threadIdx.x, nt = int64_t(gridDim.x) * blockDim.x;
+        uint4 *f4 = reinterpret_cast<uint4 *>(fin);
+        const int64_t n16 = a.n >> 4;
+        for (int64_t i = tid; i < n16; i += nt) f4[i] = make_uint4(0, 0, 0, 0);
+        for (int64_t i = (n16 << 4) + tid; i < a.n; i += nt) fin[i] = 0;
+      }
       if (!grid_barrier(rs, ++epoch, a.timeout_ns)) return;
     }
   }
