@@ -717,7 +717,7 @@ rak_status run_resident(rak_ctx *ctx, rak_graph *gr, const uint32_t *q, const ui
   a.iters = r.iters; a.start_iter = r.start; a.tolerance = r.tol; a.pickless_step = r.pickless;
   a.check_on_pickless = r.check_on_pickless; a.rescan = r.rescan; a.mark_test = rak::mark_test_for(a.n, gr->m); a.gpu_rule = r.rule == 2; a.alt = rak::alt_for(r.slots, r.mode, a.gpu_rule, false, n, gr->m, gr->ly, gr->rg); a.timeout_ns = r.timeout_ns; a.tie_until = r.tie_until; a.stage = r.stage; a.grid_cap = r.max_blocks;
   a.dense_moved_edges = rak::dense_threshold(r.mode, r.dense_pct, gr->m);
-  a.pull = rak::pull_for(r.mode, r.iters, gr->m); a.all_flags = flags == nullptr;
+  a.pull = rak::pull_for(r.mode, r.iters, gr->m, !q && !flags);
   if (renum) {
     a.off = gr->rn_off.p; a.tgt = gr->rn_tgt.as<uint32_t>(); a.wt = gr->wt ? gr->rn_wt.as<float>() : nullptr;
     a.order = gr->rn_ident.as<uint32_t>();
@@ -1417,7 +1417,7 @@ rak_status batch_enqueue(rak_ctx *ctx, rak_batch *b, const uint32_t *q, const Re
     a.running = b->running.as<unsigned int>(); a.ngraphs = G; a.grid_cap = grid_cap > 0 ? grid_cap : r.max_blocks;
     a.iters = r.iters; a.start_iter = r.start; a.tolerance = r.tol; a.pickless_step = r.pickless;
     a.check_on_pickless = r.check_on_pickless; a.rescan = r.rescan; a.mark_test = rak::mark_test_for_batch(a.n, gr->m, G); a.gpu_rule = r.rule == 2; a.alt = rak::alt_for(r.slots, r.mode, a.gpu_rule, true, n, gr->m, gr->ly, gr->rg); a.timeout_ns = r.timeout_ns; a.tie_until = r.tie_until; a.stage = r.stage;
-    a.pull = rak::pull_for(r.mode, r.iters, gr->m); a.all_flags = 1;
+    a.pull = rak::pull_for(r.mode, r.iters, gr->m, !q);
     if (a.pull) RAK_TRY(ctx, rak::launch_symmetry(gr->off, true, gr->tgt, n, gr->m, a.gid, a.vbase, rb.rs.p, st));
     int grid = 0;
     RAK_TRY(ctx, rak::launch_lpa(a, r.slots, r.mode, true, st, &grid, true));

@@ -172,13 +172,18 @@ struct LpaArgs {
   // vertex) when the previous iteration's moved vertices hold at least this many edges; 0: never
   unsigned long long dense_moved_edges;
   // synchronous modes: k_symmetry has run before the launch, so iterations may find their active set by
-  // looking for neighbours that moved (lpa_run); all_flags: every vertex starts affected
-  int pull, all_flags;
+  // looking for neighbours that moved (lpa_run); the run starts from identity labels (pull_for)
+  int pull;
   int alt;    // the other kernel of the mode (alt_for)
 };
 
-// Whether a run asks k_symmetry for that: it needs a second iteration to gain anything.
-inline int pull_for(int mode, int iters, int64_t m) { return mode != 0 && iters > 1 && m > 0 ? 1 : 0; }
+// Whether a run asks k_symmetry for that. fresh: no initial labels and no initial flags were given -- every
+// vertex starts affected and alone, and nearly every one with an edge moves. Given labels or flags mostly continue
+// a run that has settled: few vertices move, and a pass over all edges for k_symmetry, and another to find that
+// almost no neighbour moved, is more than the run itself. Measured on B200, 4.25 M vertices in cliques, synchronous
+// split, marked / pulled whatever is given: from settled labels 0.19 / 0.43 ms, with 200 vertices astray 0.25 / 0.60
+// ms, those and their flags given 0.12 / 0.36 ms. A second iteration is needed to gain anything.
+inline int pull_for(int mode, int iters, int64_t m, bool fresh) { return mode != 0 && iters > 1 && m > 0 && fresh ? 1 : 0; }
 
 enum Mode { MODE_ASYNC = 0, MODE_SYNC = 1, MODE_SPLIT = 2 };
 

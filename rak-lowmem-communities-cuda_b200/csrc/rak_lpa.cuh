@@ -1405,8 +1405,7 @@ __device__ __noinline__ Counters wide_items(const LpaArgs &a, const Regions &rg,
   } while (0)
 
 // Whether iteration it + 1 records its movers for the one after it: when the vertices that moved in
-// iteration it hold a quarter of the edges or more (in the first iteration: when every vertex starts
-// affected), and no list of region 1 that one warp would read to its end in vain is as long as to outlast the
+// iteration it hold a quarter of the edges or more (the first iteration always does, pull_for), and no list of region 1 that one warp would read to its end in vain is as long as to outlast the
 // iteration: L edges take L / 256 round trips of about half a microsecond, a balanced iteration m / 250 G/s, so
 // L up to m / 512. (Split vertices are searched by all their chunks' warps, hub_pull; the lists of smaller groups
 // are 16 * lane_max edges at most.) Measured on B200, 10 iterations of a settled vertex of 60000 edges beside
@@ -1476,7 +1475,7 @@ __global__ void __launch_bounds__(256, RAK_MIN_BLOCKS) lpa_run(const __grid_cons
     }
     if constexpr (MODE != MODE_ASYNC) {
       ph.pull_in = ph.pull_out;
-      ph.pull_out = it == 0 ? can_pull && a.iters > 1 && a.all_flags != 0 : next_out;
+      ph.pull_out = it == 0 ? can_pull : next_out;
     }
     __syncthreads();
     const int l = a.start_iter + it;

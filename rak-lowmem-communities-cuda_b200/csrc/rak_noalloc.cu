@@ -299,7 +299,7 @@ extern "C" rak_status rak_lowmem_cuda_noalloc(int device, void *stream, const ra
   a.grid_cap = o->max_blocks > 0 ? o->max_blocks : 0;
   a.timeout_ns = o->wait_timeout_ns > 0 ? (long long)o->wait_timeout_ns : DEFAULT_WAIT_TIMEOUT_NS;
   a.dense_moved_edges = dense_threshold(mode, o->dense_pct, g->m);
-  a.pull = pull_for(mode, iters, g->m); a.all_flags = o->initial_flags == nullptr;
+  a.pull = pull_for(mode, iters, g->m, !q && !o->initial_flags);
   if (a.pull) NA_TRY(launch_symmetry(g->offsets, off64, g->targets, n, g->m, nullptr, nullptr, rs, st));
   if (iters > 0) {
     int grid = 0;
