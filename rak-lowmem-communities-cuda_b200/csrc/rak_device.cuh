@@ -259,7 +259,7 @@ struct RunState {
   unsigned int error;       // rak_status of the failure
   unsigned int iterations;  // iterations performed
   unsigned long long asym;  // k_symmetry's sum: 0 for a symmetric graph
-  unsigned int pad[2];
+  unsigned int oneway, pad; // k_symmetry has met an edge that lacks its reverse, and stopped
   struct { unsigned int epoch, pad[7]; } release[BAR_FLAGS];   // the last barrier completed, one per 32-byte sector
 };
 static_assert(sizeof(RunState) == RUN_STATE_BYTES, "RunState fills the buffer the host allocates");

@@ -239,8 +239,9 @@ inline int mark_test_for_batch(int64_t n, int64_t m, int64_t graphs) {
   return graphs > 0 ? mark_test_for(n / graphs, m / graphs) : 0;
 }
 // Adds to rs->asym (RunState) a sum that is zero if every edge (u, v) has its reverse: each edge adds a
-// 64-bit hash of its unordered pair, positive from the smaller end, negative from the larger. gid, vbase:
-// the graphs of a batch (local targets), or null.
+// 64-bit hash of its unordered pair, positive from the smaller end, negative from the larger. On large graphs
+// edges are tried first, and one without its reverse sets rs->oneway and ends the pass. gid, vbase: the graphs
+// of a batch (local targets), or null.
 cudaError_t launch_symmetry(const void *off, bool off64, const uint32_t *tgt, int64_t n, int64_t m, const uint32_t *gid,
                             const int64_t *vbase, void *rs, cudaStream_t st);
 // Loads and resolves the kernel a run will launch (outside its timed region).

@@ -1462,7 +1462,7 @@ __global__ void __launch_bounds__(256, RAK_MIN_BLOCKS) lpa_run(const __grid_cons
   // moved vertex's edges plus a random flag access per edge. Decided from the previous iteration's
   // counter, which every block reads after the barrier, so all blocks agree.
   Phase ph{false, false, false, false};
-  const bool can_pull = MODE != MODE_ASYNC && a.pull != 0 && __ldcg(&rs->asym) == 0ull;
+  const bool can_pull = MODE != MODE_ASYNC && a.pull != 0 && __ldcg(&rs->asym) == 0ull && __ldcg(&rs->oneway) == 0u;
   bool next_out = false;   // whether the next iteration records its movers (Phase::pull_out)
   for (int it = 0; it < a.iters; ++it) {
     if (threadIdx.x < 4) blk[threadIdx.x] = 0;
