@@ -1,4 +1,8 @@
 // rak_kernels.cu -- plan building, validation, initialisation and FP64 modularity kernels.
+#include <sys/random.h>
+#include <time.h>
+#include <unistd.h>
+
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
 
@@ -400,7 +404,8 @@ constexpr int SYM_BATCH = 8, SYM_LIST = 64, SYM_EACH = 64;
 constexpr int64_t SYM_TRY = int64_t(1) << 22;
 template <class O, bool BATCH>
 __global__ void __launch_bounds__(TPB) k_symmetry(const O *off, const uint32_t *tgt, int64_t n, int64_t m,
-                                                  const uint32_t *gid, const int64_t *vbase, RunState *rs) {
+                                                  const uint32_t *gid, const int64_t *vbase, uint64_t key,
+                                                  RunState *rs) {
   const int lane = threadIdx.x & 31;
   const int64_t w = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5, nw = (int64_t(gridDim.x) * blockDim.x) >> 5;
   if (m >= SYM_TRY && w % SYM_EACH == 0) {
@@ -448,7 +453,7 @@ __global__ void __launch_bounds__(TPB) k_symmetry(const O *off, const uint32_t *
           if (__shfl_sync(FULL, rb, pos + s) <= at) pos += s;
         const uint32_t u = uint32_t(ub + pos), v = t[j] + (BATCH ? __shfl_sync(FULL, base, pos) : 0u);
         if (at < len && u != v) {
-          const unsigned long long h = mix64(uint64_t(u < v ? u : v) << 32 | (u < v ? v : u));
+          const unsigned long long h = mix64((uint64_t(u < v ? u : v) << 32 | (u < v ? v : u)) ^ key);
           acc += u < v ? h : 0ull - h;
         }
       }
@@ -782,15 +787,32 @@ static int edge_blocks(int64_t n, int64_t m) {
   return int(g > 148 * 8 ? 148 * 8 : (g < 1 ? 1 : g));
 }
 
+// The key of k_symmetry's hash, drawn once per process. A fixed hash would let a graph be built whose one-way edges
+// cancel in the sum (four of them are found in half a minute); with a key that the graph's maker cannot know, the sum
+// of an asymmetric graph is zero with a probability of about 2^-64. Labels do not depend on it.
+static uint64_t symmetry_key() {
+  static const uint64_t key = [] {
+    uint64_t x = 0;
+    if (getrandom(&x, sizeof x, GRND_NONBLOCK) != ssize_t(sizeof x)) {
+      timespec t{};
+      clock_gettime(CLOCK_MONOTONIC, &t);
+      x = mix64(uint64_t(t.tv_sec) << 32 ^ uint64_t(t.tv_nsec)) ^ mix64(uint64_t(getpid()) << 32 ^ reinterpret_cast<uintptr_t>(&x));
+    }
+    return mix64(x);
+  }();
+  return key;
+}
+
 cudaError_t launch_symmetry(const void *off, bool off64, const uint32_t *tgt, int64_t n, int64_t m, const uint32_t *gid,
                             const int64_t *vbase, void *rs, cudaStream_t st) {
   if (m <= 0) return cudaSuccess;
   RunState *s = static_cast<RunState *>(rs);
   const int g = edge_blocks(n, m);
+  const uint64_t key = symmetry_key();
   const int64_t *o64 = static_cast<const int64_t *>(off);
-  if (gid) k_symmetry<int64_t, true><<<g, TPB, 0, st>>>(o64, tgt, n, m, gid, vbase, s);   // batches have 64-bit offsets
-  else if (off64) k_symmetry<int64_t, false><<<g, TPB, 0, st>>>(o64, tgt, n, m, gid, vbase, s);
-  else k_symmetry<int32_t, false><<<g, TPB, 0, st>>>(static_cast<const int32_t *>(off), tgt, n, m, gid, vbase, s);
+  if (gid) k_symmetry<int64_t, true><<<g, TPB, 0, st>>>(o64, tgt, n, m, gid, vbase, key, s);   // batches have 64-bit offsets
+  else if (off64) k_symmetry<int64_t, false><<<g, TPB, 0, st>>>(o64, tgt, n, m, gid, vbase, key, s);
+  else k_symmetry<int32_t, false><<<g, TPB, 0, st>>>(static_cast<const int32_t *>(off), tgt, n, m, gid, vbase, key, s);
   return cudaGetLastError();
 }
 
