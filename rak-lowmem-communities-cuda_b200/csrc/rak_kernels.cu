@@ -202,7 +202,7 @@ __global__ void k_init_flags(uint8_t *f0, uint8_t *f1, const uint8_t *f, int64_t
 // one warp per row instead, the lanes beyond a row's degree idle, a hub is one warp's alone, and every
 // vertex adds to its community's total in memory: where one community holds most vertices those adds
 // queue on one address. Here a row's part of its total is counted (unit weights) or taken from
-// prefix sums, and the warp keeps the sum of the label it meets most in a register. Measured on B200,
+// prefix sums of the row, and the warp keeps the sum of the label it meets most in a register. Measured on B200,
 // this kernel against one warp per row: R-MAT scale 22 ef 16 0.40 ms (whole call 2.5 -> 1.1 ms; the gather
 // alone, edges read evenly, 0.37 ms), scale 24 1.75 ms (9.5 -> 3.1 ms a call), lattice 2^25 10.5 -> 2.5 ms
 // a call; all vertices in one community: lattice 2^25 54 -> 2.5 ms.
@@ -321,17 +321,18 @@ __global__ void __launch_bounds__(TPB) k_mod_edges(const O *off, const uint32_t 
               run += p;
               continue;
             }
-            // inclusive prefix sums of the 32 weights; each row takes the part between its bounds
+            // inclusive prefix sums of the 32 weights, begun anew in each row, so that a row's total holds no
+            // other row's weights; each row takes its last edge's
+            const int g0 = at - lane;
+            const int first = __shfl_sync(FULL, rb, pos) - g0;   // where this edge's row begins among the 32
 #pragma unroll
             for (int s = 1; s < 32; s <<= 1) {
               const double q = __shfl_up_sync(FULL, p, s);
-              if (lane >= s) p += q;
+              if (lane >= s && lane - s >= first) p += q;
             }
-            const int g0 = at - lane;
             const int hi = re - g0, lo = rb - g0;   // this lane's row within the 32 edges
             const double ph = __shfl_sync(FULL, p, hi >= 32 ? 31 : (hi < 1 ? 0 : hi - 1));
-            const double pl = __shfl_sync(FULL, p, lo >= 32 ? 31 : (lo < 1 ? 0 : lo - 1));
-            if (hi > 0 && lo < 32 && hi > lo) kw += ph - (lo > 0 ? pl : 0.0);
+            if (hi > 0 && lo < 32 && hi > lo) kw += ph;
           }
         }
 #pragma unroll
