@@ -70,6 +70,7 @@ struct Tracker {
 struct Arena {
   char *base = nullptr;
   size_t size = 0, used = 0;
+  bool kept = false;   // the context's scratch: counted whole by the calls that report what they hold
   static size_t rounded(size_t b) { return ((b ? b : 16) + 255) / 256 * 256; }
   bool fits(size_t b) const { return base && used + rounded(b) <= size; }
   void *take(size_t b) {
@@ -131,6 +132,7 @@ struct DevBuf {
     if (ar && ar->fits(bytes)) {
       p = ar->take(bytes);
       carved = true;
+      if (ar->kept) t = nullptr;
       if (t) t->add(bytes);
       return cudaSuccess;
     }
@@ -297,6 +299,7 @@ struct ArenaScope {
       }
       arena.base = static_cast<char *>(ctx->scratch);
       arena.size = ctx->scratch_bytes;
+      arena.kept = true;
     } else {
       if (cudaMalloc(&own, bytes) == cudaSuccess) { arena.base = static_cast<char *>(own); arena.size = bytes; }
       else { own = nullptr; cudaGetLastError(); }
@@ -310,6 +313,12 @@ struct ArenaScope {
     if (own) cudaFree(own);
   }
 };
+// Device memory a call held at its peak: what its buffers took (peak), the part of its own block that none of
+// them used, and the scratch the context keeps. given: the caller's arrays.
+uint64_t held_bytes(const rak_ctx *ctx, uint64_t peak, uint64_t given, const ArenaScope *block) {
+  const size_t size = block && block->own ? block->arena.size : 0, unused = size ? size - block->arena.used : 0;
+  return std::max<uint64_t>(peak + unused, given + size) + ctx->scratch_bytes;
+}
 size_t arena_of(std::initializer_list<size_t> buffers) {
   size_t b = 0;
   for (size_t x : buffers) b += rak_host_detail::Arena::rounded(x);
@@ -1000,7 +1009,7 @@ rak_status rak_graph_run(rak_ctx *ctx, rak_graph *gr, const uint32_t *q, const r
   RAK_CHECK(run_resident(ctx, gr, q, o ? o->initial_flags : nullptr, r, membership, &tr, rr));
   if (r.modularity)
     RAK_CHECK(modularity_dev(ctx, gr->off, gr->off64, gr->tgt, gr->wt, gr->n, gr->m, membership, &tr, &rr->modularity));
-  rr->peak_device_bytes = tr.peak + size_t(gr->n) * 4;
+  rr->peak_device_bytes = held_bytes(ctx, tr.peak + size_t(gr->n) * 4, 0, nullptr);
   return RAK_OK;
 }
 
@@ -1031,7 +1040,7 @@ rak_status rak_lowmem_cuda(rak_ctx *ctx, const rak_csr *g, const uint32_t *q, co
   if (g->location == RAK_DEVICE) {
     RAK_CHECK(run_resident(ctx, gr, q, flags, r, membership, &tr, rr));
     if (r.modularity) RAK_CHECK(modularity_dev(ctx, gr->off, gr->off64, gr->tgt, gr->wt, n, gr->m, membership, &tr, &rr->modularity));
-    rr->peak_device_bytes = tr.peak;
+    rr->peak_device_bytes = held_bytes(ctx, tr.peak, gr->ref_bytes, &arena);
     return RAK_OK;
   }
   DevBuf labels, qd, fd;
@@ -1056,7 +1065,7 @@ rak_status rak_lowmem_cuda(rak_ctx *ctx, const rak_csr *g, const uint32_t *q, co
   cudaEventRecord(ev.e[3], ctx->stream);
   RAK_TRY(ctx, cudaStreamSynchronize(ctx->stream));
   rr->d2h_ms = ev.ms(2, 3);
-  rr->peak_device_bytes = tr.peak;
+  rr->peak_device_bytes = held_bytes(ctx, tr.peak, 0, &arena);
   return RAK_OK;
 }
 
