@@ -847,15 +847,19 @@ rak_status modularity_dev(rak_ctx *ctx, const void *off, bool off64, const uint3
 
 // What a one-shot run holds beside a device-located graph: the uploaded graph and labels (host graphs), the
 // plan with its sort space, the run's buffers and, where asked for, the reference order and the modularity's
-// sums. Split vertices are counted at most.
+// sums. Split vertices are counted at most, where that is less than a label array: chunks of 32 edges would
+// take 2 bytes an edge in case there are any. Where it is more, and there are, their tables are allocated alone.
 size_t one_shot_arena(const rak_csr *g, const uint32_t *q, const rak_options *o, const Resolved &r) {
   const size_t n = size_t(std::max<int64_t>(g->n, 1)), m = size_t(std::max<int64_t>(g->m, 1));
   const size_t hubs = m / size_t(r.ly.hub_min + 1) + 1, chunks = m / size_t(r.ly.hub_chunk) + hubs;
   size_t sort = 0;
   if (g->n > 0) rak::plan_sort(nullptr, nullptr, nullptr, nullptr, g->n, 11, nullptr, &sort, nullptr);
-  size_t b = arena_of({4, n * 4, n * 4, n * 4, n * 4, size_t(nkeys_of(r.ly)) * 8, sort, hubs * 8, (hubs + 1) * 8, chunks * 4,
-                       n + 16, hubs * 4, hubs * 4, hubs * 4, chunks * size_t(r.slots) * 4, chunks * size_t(r.slots) * 4,
+  const size_t tables = arena_of({hubs * 8, (hubs + 1) * 8, chunks * 4, hubs * 4, hubs * 4, hubs * 4,
+                                  chunks * size_t(r.slots) * 4, chunks * size_t(r.slots) * 4});
+  size_t b = arena_of({4, n * 4, n * 4, n * 4, n * 4, size_t(nkeys_of(r.ly)) * 8, sort, n + 16,
                        size_t(std::max(r.iters, 1)) * rak::STATS_STRIDE * 8 + rak::RUN_STATE_BYTES});
+  // without split vertices a table has room for one
+  b += std::min(tables, std::max(n * 4, arena_of({8, 16, 4, 4, 4, 4, size_t(r.slots) * 4, size_t(r.slots) * 4})));
   if (r.mode != RAK_MODE_ASYNC) b += arena_of({n * 4 + 16, n + 16});
   if (r.order == 2) b += arena_of({n * 4, n * 4, rak::ref_order_scratch_bytes(g->n, 1)});
   if (r.modularity) b += arena_of({4, n * 8, 4 * 8});

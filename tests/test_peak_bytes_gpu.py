@@ -32,3 +32,23 @@ def test_kept_scratch_is_counted():
         after = calls(ctx)
     assert all(b < 1 << 20 for b in before)
     assert all(a >= 8 * n and a - b >= 8 * n - (1 << 20) for a, b in zip(after, before))
+
+
+@pytest.mark.parametrize("hub_min", [65536, 1 << 30])
+def test_small_chunks_of_no_split_vertex_take_no_room(hub_min):
+    """A one-shot call makes room for split vertices' tables before it knows of any: not for 2 bytes an edge. With
+    split vertices, more of them than it has room for, the call works all the same."""
+    g = rl.gen_rmat(14, 32, seed=3)
+    with rl.Context(0) as ctx:
+        _, usual = ctx.lowmem(g, mode=rl.MODE_SYNC_SPLIT)
+        _, small = ctx.lowmem(g, mode=rl.MODE_SYNC_SPLIT, hub_min=hub_min, hub_chunk=32)
+        # at most a label array more
+        assert small.peak_device_bytes <= usual.peak_device_bytes + 4 * g.n + 4096
+        opts = dict(mode=rl.MODE_SYNC_SPLIT, hub_min=256, hub_chunk=32)
+        labels, _ = ctx.lowmem(g, **opts)
+        import torch
+        rg, out = rl.ResidentGraph(ctx, g, **opts), torch.empty(g.n, dtype=torch.int32, device="cuda")
+        torch.cuda.synchronize()
+        rg.run(out, **opts)
+        assert np.array_equal(out.cpu().numpy().view(np.uint32), labels)
+        rg.close()
