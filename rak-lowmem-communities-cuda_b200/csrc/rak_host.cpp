@@ -42,12 +42,15 @@ struct rak_ctx {
   static constexpr size_t SCRATCH_KEEP = size_t(64) << 20;
   void *scratch = nullptr;
   size_t scratch_bytes = 0;
-  std::vector<cudaEvent_t> events;
+  // a fixed list: giving an event back allocates nothing and cannot throw
+  static constexpr int EVENTS_KEEP = 32;
+  cudaEvent_t events[EVENTS_KEEP] = {};
+  int nevents = 0;
   rak_ctx() = default;
   rak_ctx(const rak_ctx &) = delete;
   rak_ctx &operator=(const rak_ctx &) = delete;
   ~rak_ctx() {
-    for (cudaEvent_t e : events) cudaEventDestroy(e);
+    for (int i = 0; i < nevents; ++i) cudaEventDestroy(events[i]);
     if (scratch) cudaFree(scratch);
   }
 };
@@ -262,13 +265,18 @@ struct Events {
   rak_ctx *ctx;
   explicit Events(rak_ctx *c) : ctx(c) {
     for (auto &x : e) {
-      if (!ctx->events.empty()) { x = ctx->events.back(); ctx->events.pop_back(); }
-      else cudaEventCreate(&x);
+      if (ctx->nevents > 0) x = ctx->events[--ctx->nevents];
+      else if (cudaEventCreate(&x) != cudaSuccess) x = nullptr;
     }
   }
   Events(const Events &) = delete;
   Events &operator=(const Events &) = delete;
-  ~Events() { for (auto &x : e) if (x) ctx->events.push_back(x); }
+  ~Events() {
+    for (auto &x : e) {
+      if (x && ctx->nevents < rak_ctx::EVENTS_KEEP) ctx->events[ctx->nevents++] = x;
+      else if (x) cudaEventDestroy(x);
+    }
+  }
   float ms(int a, int b) const {
     float t = 0;
     cudaEventElapsedTime(&t, e[a], e[b]);
