@@ -94,15 +94,17 @@ inline void set_wide(Regions *rg, const unsigned long long *hist, const Layout &
     rg->wide_items = most > 32 * int64_t(rg->wide_len) ? rg->ibegin[2] : 0;
   }
 }
-// Whether a launch takes the other kernel of its mode (resolve_lpa_slots). Synchronous split runs: the one that
-// scans wide items -- there are some, Misra-Gries under the CPU rules, chains short enough for whole-number unit
-// weights (2^24 edges). Asynchronous runs: the faster lpa_run, for Misra-Gries on one graph of those that
-// mark_test_for names (rak_lpa_async.cuh says why not for the others).
+// Which kernel of its mode a launch takes (resolve_lpa_slots). Synchronous split runs: ALT_GPU_RULE under the GPU
+// rules, else ALT_FAST, the one that scans wide items -- there are some, Misra-Gries, chains short enough for
+// whole-number unit weights (2^24 edges). Asynchronous runs: ALT_FAST, the faster lpa_run, for Misra-Gries under the
+// CPU rules on one graph of those that mark_test_for names (rak_lpa_async.cuh says why not for the others).
+enum Alt { ALT_NONE = 0, ALT_FAST = 1, ALT_GPU_RULE = 2 };
 inline int mark_test_for(int64_t n, int64_t m);
 inline int alt_for(int slots, int mode, int gpu_rule, bool batch, int64_t n, int64_t m, const Layout &ly, const Regions &rg) {
-  if (slots < 2 || gpu_rule) return 0;
-  if (mode == 0) return !batch && mark_test_for(n, m) ? 1 : 0;
-  return mode == 2 && rg.wide_items > 0 && ly.hub_min <= (int64_t(1) << 29) && ly.hub_chunk <= (int64_t(1) << 29) ? 1 : 0;
+  if (mode == 2 && gpu_rule) return ALT_GPU_RULE;
+  if (slots < 2 || gpu_rule) return ALT_NONE;
+  if (mode == 0) return !batch && mark_test_for(n, m) ? ALT_FAST : ALT_NONE;
+  return mode == 2 && rg.wide_items > 0 && ly.hub_min <= (int64_t(1) << 29) && ly.hub_chunk <= (int64_t(1) << 29) ? ALT_FAST : ALT_NONE;
 }
 
 // Sort key of a vertex in the plan (regions in order, region 6 by degree descending);
@@ -158,7 +160,7 @@ struct LpaArgs {
   int64_t ngraphs;
   int grid_cap;                 // at most this many blocks (0: as many as fit), to share the GPU
   int mark_test;                // neighbour marking reads a flag before storing it (mark_test_for)
-  int gpu_rule;                 // synchronous split mode: the reference GPU sketch rules (else CPU)
+  int gpu_rule;                 // asynchronous runs: the reference GPU sketch rules (else CPU); split runs: ALT_GPU_RULE
   int tie_until;                // iterations l < tie_until break Misra-Gries ties by hash (CPU rules)
   int stage;                    // warp-wide edge ranges read through shared-memory tiles (bulk copies)
   int iters;
@@ -174,7 +176,7 @@ struct LpaArgs {
   // synchronous modes: k_symmetry has run before the launch, so iterations may find their active set by
   // looking for neighbours that moved (lpa_run); the run starts from identity labels (pull_for)
   int pull;
-  int alt;    // the other kernel of the mode (alt_for)
+  int alt;    // which kernel of the mode (alt_for)
 };
 
 // Whether a run asks k_symmetry for that. fresh: no initial labels and no initial flags were given -- every
@@ -220,7 +222,7 @@ cudaError_t launch_lpa(const LpaArgs &a, int slots, int mode, bool off64, cudaSt
 template <int S>
 cudaError_t launch_lpa_slots(const LpaArgs &a, int mode, bool off64, bool batch, cudaStream_t st, int *grid_out);
 template <int S>
-cudaError_t resolve_lpa_slots(int mode, bool off64, bool unit, bool batch, bool stage, bool alt, const void **fn, int *per_sm);
+cudaError_t resolve_lpa_slots(int mode, bool off64, bool unit, bool batch, bool stage, int alt, const void **fn, int *per_sm);
 // The asynchronous kernel that keeps its pace (rak_lpa_async.cuh; rak_lpa_async_s*.cu).
 template <int S>
 const void *async_kernel(bool off64, bool unit, bool batch);
@@ -245,7 +247,7 @@ inline int mark_test_for_batch(int64_t n, int64_t m, int64_t graphs) {
 cudaError_t launch_symmetry(const void *off, bool off64, const uint32_t *tgt, int64_t n, int64_t m, const uint32_t *gid,
                             const int64_t *vbase, void *rs, cudaStream_t st);
 // Loads and resolves the kernel a run will launch (outside its timed region).
-cudaError_t prepare_lpa(int slots, int mode, bool off64, bool unit, bool batch, bool stage, bool alt);
+cudaError_t prepare_lpa(int slots, int mode, bool off64, bool unit, bool batch, bool stage, int alt);
 
 // Plan and utility kernels (rak_kernels.cu).
 cudaError_t launch_validate(const void *off, bool off64, const uint32_t *tgt, int64_t n, int64_t m,

@@ -839,7 +839,7 @@ cudaError_t launch_modularity(const void *off, bool off64, const uint32_t *tgt, 
   return cudaGetLastError();
 }
 
-cudaError_t prepare_lpa(int slots, int mode, bool off64, bool unit, bool batch, bool stage, bool alt) {
+cudaError_t prepare_lpa(int slots, int mode, bool off64, bool unit, bool batch, bool stage, int alt) {
   const void *fn = nullptr;
   int per_sm = 0;
   switch (slots) {

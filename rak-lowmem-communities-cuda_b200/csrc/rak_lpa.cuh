@@ -1392,18 +1392,6 @@ __device__ __noinline__ Counters wide_items(const LpaArgs &a, const Regions &rg,
   return cnt;
 }
 
-// The rule set of a work item: the exact synchronous mode follows the CPU rules; the split-layout
-// modes (asynchronous and synchronous split) either, per launch (a.gpu_rule).
-#define RAK_BY_RULE(F, ARGS)                                                            \
-  do {                                                                                 \
-    if constexpr (MODE != MODE_SYNC) {                                                 \
-      if (a.gpu_rule) F<S, MODE, O, UNIT, BATCH, RULE_GPU> ARGS;                       \
-      else F<S, MODE, O, UNIT, BATCH, RULE_CPU> ARGS;                       \
-    } else {                                                                           \
-      F<S, MODE, O, UNIT, BATCH, RULE_CPU> ARGS;                                       \
-    }                                                                                  \
-  } while (0)
-
 // Whether iteration it + 1 records its movers for the one after it: when the vertices that moved in
 // iteration it hold a quarter of the edges or more (the first iteration always does, pull_for), and no list of region 1 that one warp would read to its end in vain is as long as to outlast the
 // iteration: L edges take L / 256 round trips of about half a microsecond, a balanced iteration m / 250 G/s, so
@@ -1419,7 +1407,9 @@ __device__ __forceinline__ bool pulls_next(const LpaArgs &a, int it, bool can_pu
 // WIDE: the launch has wide items. Launches without any take a kernel that does not hold their code and
 // shared memory (one kernel for both: R-MAT scale 24 ef 16 split 50.7 -> 52.4 ms, lattice 2047x2049 1.16 -> 1.24
 // ms). Asynchronous runs take this kernel only where their result does not show its pace (rak_lpa_async.cuh).
-template <int S, int MODE, class O, bool UNIT, bool BATCH, bool WIDE>
+// RULE: the rule set of the work items. Only split runs know both, each with a kernel of its own: the exact mode
+// follows the CPU rules, and wide items and asynchronous runs that come here do.
+template <int S, int MODE, class O, bool UNIT, bool BATCH, bool WIDE, int RULE>
 __global__ void __launch_bounds__(256, RAK_MIN_BLOCKS) lpa_run(const __grid_constant__ LpaArgs a) {
   const G_<O> g{static_cast<const O *>(a.off), a.tgt, a.wt};
   RunState *rs = static_cast<RunState *>(a.rs);
@@ -1512,7 +1502,7 @@ __global__ void __launch_bounds__(256, RAK_MIN_BLOCKS) lpa_run(const __grid_cons
           if (sub * 32 >= rg.vcount[REG_LANE]) break;
           qn = lane_collect<MODE, O, BATCH>(a, rg, g, sub, vin, vout, fin, fout, q, qn, ph);
           if (qn >= 32) {
-            RAK_BY_RULE(lane_batch, (a, g, q, 32, it, pickless, vin, vout, fin, fout, cnt, ph));
+            lane_batch<S, MODE, O, UNIT, BATCH, RULE>(a, g, q, 32, it, pickless, vin, vout, fin, fout, cnt, ph);
             __syncwarp();
             if (lane < qn - 32) q[lane] = q[32 + lane];
             __syncwarp();
@@ -1520,12 +1510,12 @@ __global__ void __launch_bounds__(256, RAK_MIN_BLOCKS) lpa_run(const __grid_cons
           }
         }
       } else if (r == REG_HUB) {
-        RAK_BY_RULE(hub_item, (a, rg, g, local, it, pickless, vin, vout, fin, fout, cnt, sc, ph));
+        hub_item<S, MODE, O, UNIT, BATCH, RULE>(a, rg, g, local, it, pickless, vin, vout, fin, fout, cnt, sc, ph);
       } else {
-        RAK_BY_RULE(group_item, (a, rg, g, r, local, it, pickless, vin, vout, fin, fout, cnt, sc, ph));
+        group_item<S, MODE, O, UNIT, BATCH, RULE>(a, rg, g, r, local, it, pickless, vin, vout, fin, fout, cnt, sc, ph);
       }
     }
-    if (qn > 0) RAK_BY_RULE(lane_batch, (a, g, q, qn, it, pickless, vin, vout, fin, fout, cnt, ph));
+    if (qn > 0) lane_batch<S, MODE, O, UNIT, BATCH, RULE>(a, g, q, qn, it, pickless, vin, vout, fin, fout, cnt, ph);
     __syncwarp();
     const unsigned long long ch = warp_sum((unsigned long long)cnt.changed);
     const unsigned long long ed = warp_sum(cnt.edges);
@@ -1635,7 +1625,7 @@ inline size_t lpa_dynamic_smem(int mode, bool unit, bool stage) {
 // device). The first query of an instantiation loads its module (CUDA loads modules lazily, which
 // can take a millisecond), so runs resolve before their timed region (prepare_lpa).
 template <int S>
-cudaError_t resolve_lpa_slots(int mode, bool off64, bool unit, bool batch, bool stage, bool alt, const void **fn_out,
+cudaError_t resolve_lpa_slots(int mode, bool off64, bool unit, bool batch, bool stage, int alt, const void **fn_out,
                               int *per_sm_out) {
   const void *fn = nullptr;
 #define RAK_PICK(M, O, U, B)                                                          \
@@ -1643,12 +1633,15 @@ cudaError_t resolve_lpa_slots(int mode, bool off64, bool unit, bool batch, bool 
     if constexpr (M == MODE_ASYNC) {                                                  \
       fn = async_kernel<S>(off64, unit, batch);                                        \
       if constexpr (S > 1 && !B) {                                                    \
-        if (alt) fn = reinterpret_cast<const void *>(&lpa_run<S, M, O, U, B, false>); \
+        if (alt) fn = reinterpret_cast<const void *>(&lpa_run<S, M, O, U, B, false, RULE_CPU>); \
       }                                                                               \
     } else {                                                                          \
-      fn = reinterpret_cast<const void *>(&lpa_run<S, M, O, U, B, false>);            \
+      fn = reinterpret_cast<const void *>(&lpa_run<S, M, O, U, B, false, RULE_CPU>);  \
+      if constexpr (M == MODE_SPLIT) {                                                \
+        if (alt == ALT_GPU_RULE) fn = reinterpret_cast<const void *>(&lpa_run<S, M, O, U, B, false, RULE_GPU>); \
+      }                                                                               \
       if constexpr (has_wide<S, M>()) {                                               \
-        if (alt) fn = reinterpret_cast<const void *>(&lpa_run<S, M, O, U, B, true>);  \
+        if (alt == ALT_FAST) fn = reinterpret_cast<const void *>(&lpa_run<S, M, O, U, B, true, RULE_CPU>); \
       }                                                                               \
     }                                                                                 \
   }
@@ -1691,14 +1684,14 @@ template <int S>
 cudaError_t launch_lpa_slots(const LpaArgs &a, int mode, bool off64, bool batch, cudaStream_t st, int *grid_out) {
   const void *fn = nullptr;
   int per_sm = 0, dev = 0, sms = 0;
-  cudaError_t e = resolve_lpa_slots<S>(mode, off64, a.wt == nullptr, batch, a.stage != 0, a.alt != 0, &fn, &per_sm);
+  cudaError_t e = resolve_lpa_slots<S>(mode, off64, a.wt == nullptr, batch, a.stage != 0, a.alt, &fn, &per_sm);
   if (e != cudaSuccess) return e;
   if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
   if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
   const int64_t warps_needed = a.rg.ibegin[NREG] > 0 ? a.rg.ibegin[NREG] : 1;
   int64_t grid = int64_t(per_sm) * sms;
   int64_t want = (warps_needed + 7) / 8;
-  if (mode == MODE_SPLIT && a.alt && a.rg.wide_items > want) want = a.rg.wide_items;   // a block each
+  if (mode == MODE_SPLIT && a.alt == ALT_FAST && a.rg.wide_items > want) want = a.rg.wide_items;   // a block each
   if (want < grid) grid = want;
   if (a.grid_cap > 0 && grid > a.grid_cap) grid = a.grid_cap;
   if (grid < 1) grid = 1;
