@@ -127,7 +127,9 @@ __device__ __forceinline__ void unit_acc(UnitSketch<S> &s, uint32_t c) {
 }
 // The weights as floats. ORDER: only their order is needed (the sketch goes straight to the argmax), so
 // the whole numbers keep their bits -- small floats in the same order, zero at zero -- and the
-// integer-to-float conversions, a quarter-rate instruction each, are saved.
+// integer-to-float conversions, a quarter-rate instruction each, are saved. Such floats are denormal, so the
+// argmax and the move rule compare them as the whole numbers they are (BITS below): a build that flushes
+// denormals (-ftz=true) would see them all as zero.
 template <int S, bool ORDER>
 __device__ __forceinline__ void unit_to_sketch(const UnitSketch<S> &u, Sketch<S> &s) {
 #pragma unroll
@@ -204,10 +206,20 @@ __device__ __forceinline__ void sk_tree(Sketch<S> &s, int G) {
   }
 }
 
+// a > b. BITS: neither is negative, so their bits compare as they do, denormal or not.
+template <bool BITS>
+__device__ __forceinline__ bool heavier(float a, float b) {
+  return BITS ? __float_as_int(a) > __float_as_int(b) : a > b;
+}
+template <bool BITS>
+__device__ __forceinline__ bool as_heavy(float a, float b) {
+  return BITS ? __float_as_int(a) == __float_as_int(b) : a == b;
+}
+
 // CPU rule: linear argmax with strict '>' from weight 0 (inc/rakLowmem.hxx:164-171).
 // GPU rule: the tournament of sketchMaxGroupReduceCudU (inc/sketchCuda.hxx:190-201) -- at each
 // level slot i takes slot i+S/2 only if strictly heavier -- whose winner may weigh <= 0.
-template <int S, int RULE = RULE_CPU>
+template <int S, int RULE = RULE_CPU, bool BITS = false>
 __device__ __forceinline__ void sk_choose(const Sketch<S> &s, uint32_t &c, float &w) {
   if constexpr (RULE == RULE_GPU) {
     uint32_t k[S];
@@ -227,7 +239,7 @@ __device__ __forceinline__ void sk_choose(const Sketch<S> &s, uint32_t &c, float
     w = 0.0f;
 #pragma unroll
     for (int i = 0; i < S; ++i)
-      if (s.w[i] > w) { w = s.w[i]; c = s.k[i]; }
+      if (heavier<BITS>(s.w[i], w)) { w = s.w[i]; c = s.k[i]; }
   }
 }
 
@@ -239,7 +251,7 @@ __device__ __forceinline__ void sk_choose(const Sketch<S> &s, uint32_t &c, float
 __host__ __device__ __forceinline__ uint64_t tie_hash(uint32_t u, uint32_t key, uint32_t l) {
   return mix64((uint64_t(key) << 32 | uint64_t(u)) ^ (uint64_t(l) * 0xD6E8FEB86659FD93ull));
 }
-template <int S>
+template <int S, bool BITS = false>
 __device__ __forceinline__ void sk_choose_hashed(const Sketch<S> &s, uint32_t u, uint32_t l, uint32_t &c, float &w) {
   c = NONE;
   w = 0.0f;
@@ -247,7 +259,7 @@ __device__ __forceinline__ void sk_choose_hashed(const Sketch<S> &s, uint32_t u,
 #pragma unroll
   for (int i = 0; i < S; ++i) {
     const uint64_t h = tie_hash(u, s.k[i], l);
-    if (s.w[i] > w || (s.w[i] == w && w > 0.0f && h > hb)) { w = s.w[i]; c = s.k[i]; hb = h; }
+    if (heavier<BITS>(s.w[i], w) || (as_heavy<BITS>(s.w[i], w) && heavier<BITS>(w, 0.0f) && h > hb)) { w = s.w[i]; c = s.k[i]; hb = h; }
   }
 }
 

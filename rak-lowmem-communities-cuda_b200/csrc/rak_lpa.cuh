@@ -776,26 +776,26 @@ __device__ __forceinline__ void count_moves(const LpaArgs &a, uint32_t gi, int i
 // CPU rule: w > 0 && c != d (inc/rakLowmem.hxx:203). GPU rule: the best weight is non-zero for
 // Misra-Gries (inc/rakLowmemCuda.hxx:306), any candidate for Boyer-Moore (:152). Both: on pickless
 // iterations no move to a larger label (:309, :153).
-template <int S, int RULE>
+template <int S, int RULE, bool BITS = false>
 __device__ __forceinline__ bool move_rule(float w, uint32_t c, uint32_t d, bool pickless) {
-  const bool weight_ok = RULE == RULE_GPU ? (S == 1 || w != 0.0f) : w > 0.0f;
+  const bool weight_ok = RULE == RULE_GPU ? (S == 1 || w != 0.0f) : heavier<BITS>(w, 0.0f);
   return weight_ok && c != d && !(pickless && c > d);
 }
 
 // Argmax of a vertex's sketch under the launch's tie rule: hashed ties on iterations
 // l < a.tie_until (Misra-Gries, CPU rules), else the rule set's own. u_local: the vertex's id within
 // its graph, so a graph breaks its ties the same way alone and in a batch.
-template <int S, int RULE>
+template <int S, int RULE, bool BITS = false>
 __device__ __forceinline__ void choose(const LpaArgs &a, const Sketch<S> &sk, uint32_t u_local, int it, uint32_t &c,
                                        float &w) {
   if constexpr (S > 1 && RULE != RULE_GPU) {
     const int l = a.start_iter + it;
     if (l < a.tie_until) {
-      sk_choose_hashed<S>(sk, u_local, uint32_t(l), c, w);
+      sk_choose_hashed<S, BITS>(sk, u_local, uint32_t(l), c, w);
       return;
     }
   }
-  sk_choose<S, RULE>(sk, c, w);
+  sk_choose<S, RULE, BITS>(sk, c, w);
 }
 
 // ---- the active set of a synchronous iteration, pulled ------------------------------------------
@@ -893,14 +893,15 @@ __device__ __forceinline__ int lane_collect(const LpaArgs &a, const Regions &rg,
 }
 
 // The choice and move of an active vertex scanned by one lane; true if it moved.
-template <int S, int MODE, bool BATCH, int RULE>
+template <int S, int MODE, bool UNIT, bool BATCH, int RULE>
 __device__ __forceinline__ bool lane_close(const LpaArgs &a, const Sketch<S> &sk, uint32_t u, uint32_t d, uint32_t gi,
                                            uint32_t base, int64_t deg, int it, bool pickless, uint32_t *vout, uint8_t *fin,
                                            uint8_t *fout, Counters &cnt, Phase ph) {
   uint32_t c;
   float w;
-  choose<S, RULE>(a, sk, u - base, it, c, w);
-  const bool moved = move_rule<S, RULE>(w, c, d, pickless);
+  constexpr bool BITS = unit_sketch<S, UNIT, RULE>();   // weights as unit_to_sketch<S, true> leaves them
+  choose<S, RULE, BITS>(a, sk, u - base, it, c, w);
+  const bool moved = move_rule<S, RULE, BITS>(w, c, d, pickless);
   cnt.processed += 1;
   cnt.edges += (unsigned long long)deg;
   if constexpr (MODE == MODE_ASYNC) {
@@ -936,7 +937,7 @@ __device__ __forceinline__ void lane_batch(const LpaArgs &a, const G_<O> &g, con
   else scan_range<S, UNIT, RULE, true>(sk, u, eb, ee, 1, g.tgt, g.wt, vin, base);
   if constexpr (MODE == MODE_SYNC && S > 1)
     if (a.rescan) rescan_range<S, UNIT>(sk, u, eb, ee, g.tgt, g.wt, vin, base);
-  if (!lane_close<S, MODE, BATCH, RULE>(a, sk, u, d, gi, base, ee - eb, it, pickless, vout, fin, fout, cnt, ph)) return;
+  if (!lane_close<S, MODE, UNIT, BATCH, RULE>(a, sk, u, d, gi, base, ee - eb, it, pickless, vout, fin, fout, cnt, ph)) return;
   if (ph.nomark || ph.pull_out) return;
   if (!vec) mark_item<S>(a, u, eb, ee, 1, g.tgt, fout, base);
   else if (mark_tested<S>(a)) mark_lane<true>(u, eb, ee, g.tgt, fout, base);
