@@ -96,14 +96,31 @@ inline void set_wide(Regions *rg, const unsigned long long *hist, const Layout &
 }
 // Which kernel of its mode a launch takes (resolve_lpa_slots). Synchronous split runs: ALT_GPU_RULE under the GPU
 // rules, else ALT_FAST, the one that scans wide items -- there are some, Misra-Gries, chains short enough for
-// whole-number unit weights (2^24 edges). Asynchronous runs: ALT_FAST, the faster lpa_run, for Misra-Gries under the
-// CPU rules on one graph of those that mark_test_for names (rak_lpa_async.cuh says why not for the others).
+// whole-number unit weights (2^24 edges). Asynchronous runs: ALT_FAST, the faster lpa_run, for those of one graph
+// under the CPU rules that async_fast names.
 enum Alt { ALT_NONE = 0, ALT_FAST = 1, ALT_GPU_RULE = 2 };
-inline int mark_test_for(int64_t n, int64_t m);
+
+// Asynchronous runs whose modularity does not depend on which kernel's pace they run at, and that are faster for
+// it: 8 slots, 2^22 vertices or more of average degree 8 or more, an eighth of the edges or more in lists above 256
+// (a lower bound of them, from the plan's regions; layouts with a lower lane_max are not measured and keep their
+// kernel). Measured on B200, 96 runs of each kernel in 3 processes, modularity of lpa_run against lpa_run_async
+// with the difference over the standard error of the processes' means, and ms a run: R-MAT scale 22 ef 16 +0.012% (3.4)
+// 3.37 -> 3.20, weighted -0.004% (-0.9) 3.67 -> 3.42, ef 32 weighted -0.023% (-1.3) 10.0 -> 9.3, scale 23 +0.008%
+// (2.6) 5.87 -> 5.49, scale 24 +0.009% (7.4) 11.4 -> 10.6, R-MAT of flatter quadrants (0.45, 0.22) +0.001% (2.8) 4.66 ->
+// 4.53. Elsewhere it is lower or not faster: 16 slots R-MAT scale 22 -0.12%, 2 slots -0.08%, 4 slots scale 23 -0.04%
+// (5.44 -> 5.35 ms); 8 slots, lattice of 12 neighbours and 4.2 M vertices -1.7%; SBM of 4.2 M vertices +0.003%, 2.30 ->
+// 2.28 ms.
+inline bool async_fast(int slots, int64_t n, int64_t m, const Layout &ly, const Regions &rg) {
+  if (slots != 8 || n < (int64_t(1) << 22) || m < 8 * n || ly.lane_max < DEFAULT_LANE_MAX) return false;
+  int64_t edges = rg.vcount[0] * ly.hub_min;
+  for (int r = 1; r < REG_LANE; ++r) edges += rg.vcount[r] * ((ly.lane_max * region_group(r)) >> 1);
+  return edges >= m / 8;
+}
+
 inline int alt_for(int slots, int mode, int gpu_rule, bool batch, int64_t n, int64_t m, const Layout &ly, const Regions &rg) {
   if (mode == 2 && gpu_rule) return ALT_GPU_RULE;
   if (slots < 2 || gpu_rule) return ALT_NONE;
-  if (mode == 0) return !batch && mark_test_for(n, m) ? ALT_FAST : ALT_NONE;
+  if (mode == 0) return !batch && async_fast(slots, n, m, ly, rg) ? ALT_FAST : ALT_NONE;
   return mode == 2 && rg.wide_items > 0 && ly.hub_min <= (int64_t(1) << 29) && ly.hub_chunk <= (int64_t(1) << 29) ? ALT_FAST : ALT_NONE;
 }
 

@@ -5,9 +5,8 @@
 // rules at another pace ended at another modularity, by several times what runs of one kernel differ by --
 // even where only the order of instructions had changed (eight lattices of 2047x2049: 0.6592 +- 0.0002
 // against 0.6569 to 0.6604; SBM of 300 k vertices 0.1043 +- 0.0001 against 0.1032 to 0.1051). These runs keep
-// their first kernel, with its scan, accumulate and barrier. Misra-Gries on single graphs of 2^22 vertices and
-// average degree 8 or more (mark_test_for) takes the faster lpa_run (rak_lpa.cuh): there the pace does not
-// show (R-MAT scale 22 0.03304 and 0.03304, weighted 0.02812 and 0.02812).
+// their first kernel, with its scan, accumulate and barrier. Runs with 8 slots on large skewed graphs (async_fast,
+// with the measurements) take the faster lpa_run (rak_lpa.cuh): there the pace does not show.
 //
 // Work items, phases and rules as described in rak_lpa.cuh. Compiled in units of its own, with the compiler's
 // default scheme: splitting the compilation (the Makefile's flag for the other units) orders the instructions
@@ -178,11 +177,10 @@ __device__ __forceinline__ void async_group_item(const LpaArgs &a, const Regions
   if (moved && !ph.nomark) mark_item<S>(a, u, eb + s, ee, G, g.tgt, fout, base);
 }
 
-// Region 0: one chunk of a split vertex per item. In the synchronous exact mode chunk 0's warp
-// scans the whole vertex in edge order and the other chunks do nothing. Otherwise each chunk's
-// warp builds a partial sketch (lane-strided, tree-merged), stores it, and the last chunk to
-// arrive merges all partial sketches in a fixed order and makes the move; its neighbours are
-// marked in a second phase after the iteration's barrier.
+// Region 0: one chunk of a split vertex per item. Each chunk's warp builds a partial sketch
+// (lane-strided, tree-merged), stores it, and the last chunk to arrive merges all partial sketches
+// in a fixed order and makes the move; its neighbours are marked in a second phase after the
+// iteration's barrier.
 template <int S, class O, bool UNIT, bool BATCH, int RULE>
 __device__ __forceinline__ void async_hub_item(const LpaArgs &a, const Regions &rg, const G_<O> &g, int64_t local, int it, bool pickless,
                                          const uint32_t *vin, uint32_t *vout, uint8_t *fin, uint8_t *fout,
