@@ -158,7 +158,7 @@ __device__ __forceinline__ void scan_edges(ACC &&acc, uint32_t u, int64_t e, int
   constexpr int B = RAK_SCAN_BATCH;
   // edges of this lane: a chain is at most hub_min / 32, hub_chunk / 32 or lane_max edges, so an int holds
   // it, and 32-bit counts keep the 64-bit address arithmetic to one add per stage
-  int left = int((ee - e + st - 1) / st);
+  int left = int((ee - e + st - 1) >> (31 - __clz(st)));   // st: a power of two
   const uint32_t *tp = tgt + e;
   const float *wp = UNIT ? nullptr : wt + e;
   uint32_t t[B], t1[B], c[B];
@@ -1019,8 +1019,10 @@ __device__ __forceinline__ void group_item(const LpaArgs &a, const Regions &rg, 
   Sketch<S> sk;
   sk_clear<S, RULE>(sk, v.d);
   if constexpr (MODE == MODE_SYNC) {
-    // groups of 8 lanes or more (1024 edges or more): their lists one after the other by the whole warp; smaller
-    // groups side by side (lists one after the other from 2 lanes on: R-MAT scale 12 without rescan 2.0 -> 3.5 ms)
+    // groups of 8 lanes or more (lists above 4 * lane_max edges, 1024 by default): their lists one after the other
+    // by the whole warp; smaller groups side by side (lists one after the other from 2 lanes on: R-MAT scale 12 without
+    // rescan 2.0 -> 3.5 ms). With a small lane_max the same line pays: lane_max 8, lists of 33 edges or more, edge by
+    // edge -> this, degree 34 1.80 -> 1.47 ms, degree 64 4.85 -> 2.46 ms, R-MAT scale 14 6.6 -> 1.57 ms
     if (S > 1 && G >= 8) {
       for (int o = 0; o < 32; o += G) {
         if (__shfl_sync(FULL, int(v.active), o) == 0) continue;
@@ -1065,9 +1067,9 @@ struct HubChunk {
 // launches use otherwise) takes the iteration's number. Each edge is looked at once at most, by as many warps as
 // there are chunks; a search of the whole list by every chunk's warp instead made a settled vertex of a million
 // edges beside moving ones cost 12 ms an iteration (R-MAT graphs, whose first edges find a mover: the same). The
-// caller's barrier comes before and after. A function of its own, not inlined, as wide_items.
+// caller's barrier comes before and after. Inlined: as a function of its own it cost batches 4%.
 template <class O, bool BATCH>
-__device__ __noinline__ void hub_pull(const LpaArgs &a, const Regions &rg, const uint8_t *movers, int next) {
+__device__ __forceinline__ void hub_pull(const LpaArgs &a, const Regions &rg, const uint8_t *movers, int next) {
   const G_<O> g{static_cast<const O *>(a.off), a.tgt, a.wt};
   const int lane = threadIdx.x & 31;
   const int64_t gw = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;

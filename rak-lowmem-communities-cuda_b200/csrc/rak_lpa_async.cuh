@@ -8,9 +8,9 @@
 // their first kernel, with its scan, accumulate and barrier. Runs with 8 slots on large skewed graphs (async_fast,
 // with the measurements) take the faster lpa_run (rak_lpa.cuh): there the pace does not show.
 //
-// Work items, phases and rules as described in rak_lpa.cuh. Compiled in units of its own, with the compiler's
-// default scheme: splitting the compilation (the Makefile's flag for the other units) orders the instructions
-// differently, which shows in the result as above.
+// Work items, phases and rules as described in rak_lpa.cuh. Compiled in units of its own, and none of the library's
+// with a split compilation (--split-compile), which orders the instructions differently: here it shows in the
+// result as above.
 #pragma once
 #include "rak_lpa.cuh"
 
