@@ -822,9 +822,9 @@ rak_status run_resident(rak_ctx *ctx, rak_graph *gr, const uint32_t *q, const ui
       res->traversed_edges += st_i[rak::STAT_EDGES];
       res->processed_vertices += st_i[rak::STAT_PROCESSED];
       res->moved_vertices += st_i[rak::STAT_CHANGED];
-      res->moved_edges += st_i[rak::STAT_MOVED_EDGES];
+      res->moved_edges += rak::moved_edges(st_i);
       if (st_i[rak::STAT_PHASE] & 1ull) res->dense_iterations += 1;
-      else res->marked_edges += st_i[rak::STAT_MOVED_EDGES];
+      else res->marked_edges += rak::moved_edges(st_i);
     }
     res->changed_last = done > 0 ? stats[size_t(done - 1) * rak::STATS_STRIDE + rak::STAT_CHANGED] : 0;
     res->memory_gb = float(double(b.bytes() + size_t(n) * 4 + gr->plan_bytes + (renum ? gr->rn_bytes() : 0)) /
@@ -1563,8 +1563,8 @@ rak_status rak_batch_results(rak_ctx *ctx, rak_batch *b, int32_t *iterations, ra
       total->traversed_edges += x[rak::STAT_EDGES];
       total->processed_vertices += x[rak::STAT_PROCESSED];
       total->moved_vertices += x[rak::STAT_CHANGED];
-      total->moved_edges += x[rak::STAT_MOVED_EDGES];
-      total->marked_edges += x[rak::STAT_MOVED_EDGES];   // batches mark after every move
+      total->moved_edges += rak::moved_edges(x);
+      total->marked_edges += rak::moved_edges(x);   // batches mark after every move
     }
     total->changed_last = done > 0 ? st[size_t(done - 1) * rak::STATS_STRIDE + rak::STAT_CHANGED] : 0;
     total->plan_ms = b->g->plan_ms;

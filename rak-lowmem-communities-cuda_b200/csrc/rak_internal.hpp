@@ -225,10 +225,13 @@ inline int default_label_order(int mode, int slots) { return mode == MODE_ASYNC 
 
 // Per-iteration counters written by the LPA kernel.
 // STAT_PHASE: how the iteration treated the frontier (bit 0: its moves marked no neighbours; bit 1:
-// it processed every vertex), written by the asynchronous single-graph kernel. STAT_IDLE: the same word in the
-// synchronous modes, from bit 1 on the longest list of region 1 that was not in the active set.
+// it processed every vertex), written by the asynchronous single-graph kernel.
 enum Stat { STAT_CHANGED = 0, STAT_EDGES = 1, STAT_PROCESSED = 2, STAT_HUBS_MOVED = 3, STAT_MOVED_EDGES = 4, STAT_WORK = 5,
-            STAT_PHASE = 6, STAT_IDLE = 6, STAT_WIDE = 7 };
+            STAT_PHASE = 6, STAT_WIDE = 7 };
+// In STAT_MOVED_EDGES of a synchronous iteration: a list of region 1 longer than m / 512 was not in the active set.
+// In the same word, for the kernel reads both in every iteration; moved_edges leaves it out.
+constexpr unsigned long long LONG_IDLE = 1ull << 63;
+inline unsigned long long moved_edges(const unsigned long long *iteration) { return iteration[STAT_MOVED_EDGES] & ~LONG_IDLE; }
 constexpr int STATS_STRIDE = 8;
 
 // Persistent cooperative launch of all iterations; grid chosen from occupancy. `batch` selects the

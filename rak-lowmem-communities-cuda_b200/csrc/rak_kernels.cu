@@ -398,11 +398,11 @@ __global__ void __launch_bounds__(TPB) k_mod_edges(const O *off, const uint32_t 
 // the targets with a 64-bit mix per edge, bound by its instructions: 320 G edges/s (R-MAT scale 22 ef 16 0.40 ms, SBM of
 // 4 M vertices 0.23 ms). On graphs of SYM_TRY edges or more every SYM_EACH-th warp first tries 32 vertices:
 // whether the list of the first neighbour, if it has SYM_LIST edges or fewer, holds the reverse. Directed graphs
-// end there (32 M one-way edges: 0.02 ms), graphs that lack a few reverse edges pay the pass. On smaller graphs the
-// pass is about as short as the trial; and a few warps try, since each that finds an edge stores to the one word
+// end there (32 M one-way edges: 0.02 ms), graphs that lack a few reverse edges pay the pass. Below that the pass
+// takes 0.05 ms or less, and the trial would add to it on every symmetric graph; and a few warps try, since each that finds an edge stores to the one word
 // that all look at, and such stores take each other's turn (every warp trying: 0.28 ms).
 constexpr int SYM_BATCH = 8, SYM_LIST = 64, SYM_EACH = 64;
-constexpr int64_t SYM_TRY = int64_t(1) << 22;
+constexpr int64_t SYM_TRY = int64_t(1) << 24;
 template <class O, bool BATCH>
 __global__ void __launch_bounds__(TPB) k_symmetry(const O *off, const uint32_t *tgt, int64_t n, int64_t m,
                                                   const uint32_t *gid, const int64_t *vbase, uint64_t key,

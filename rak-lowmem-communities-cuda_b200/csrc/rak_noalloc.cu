@@ -330,9 +330,9 @@ extern "C" rak_status rak_lowmem_cuda_noalloc(int device, void *stream, const ra
     rr->traversed_edges += x[STAT_EDGES];
     rr->processed_vertices += x[STAT_PROCESSED];
     rr->moved_vertices += x[STAT_CHANGED];
-    rr->moved_edges += x[STAT_MOVED_EDGES];
+    rr->moved_edges += moved_edges(x);
     if (x[STAT_PHASE] & 1ull) rr->dense_iterations += 1;
-    else rr->marked_edges += x[STAT_MOVED_EDGES];
+    else rr->marked_edges += moved_edges(x);
   }
   rr->changed_last = done > 0 ? sh[size_t(done - 1) * STATS_STRIDE + STAT_CHANGED] : 0;
   rr->peak_device_bytes = cv.need;

@@ -55,7 +55,7 @@ def _star_and_pairs(leaves, one_way):
 @pytest.mark.parametrize("mode", [rl.MODE_SYNC, rl.MODE_SYNC_SPLIT])
 def test_settled_list_beside_moving_pairs(ctx, leaves, mode):
     import torch
-    ms, labels, moved = [], [], []
+    ms, labels, moved, edges = [], [], [], []
     for one_way in (False, True):
         g = _star_and_pairs(leaves, one_way)
         rg = rl.ResidentGraph(ctx, g, mode=mode)
@@ -69,8 +69,10 @@ def test_settled_list_beside_moving_pairs(ctx, leaves, mode):
         ms.append(min(took))
         labels.append(out.cpu().numpy()[:g.n - 2])
         moved.append(r.moved_vertices)
+        edges.append(r.moved_edges)
     assert np.array_equal(labels[0], labels[1])
     assert moved[0] in (moved[1], moved[1] - 1)   # the one-way edge moves its vertex once
+    assert edges[0] in (edges[1], edges[1] - 1)
     # 30 iterations; 0.2 ms: the grid barriers and launch jitter of either side
     assert ms[0] <= 3 * ms[1] + 0.2, ms
 
