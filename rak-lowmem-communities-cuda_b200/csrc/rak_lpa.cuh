@@ -1403,12 +1403,15 @@ __device__ __noinline__ Counters wide_items(const LpaArgs &a, const Regions &rg,
 }
 
 // Whether iteration it + 1 records its movers for the one after it: when the vertices that moved in
-// iteration it hold a quarter of the edges or more (the first iteration always does, pull_for), and no list of region 1 that one warp would read to its end in vain is as long as to outlast the
-// iteration: L edges take L / 256 round trips of about half a microsecond, a balanced iteration m / 250 G/s, so
-// L up to m / 512. (Split vertices are searched by all their chunks' warps, hub_pull; the lists of smaller groups
-// are 16 * lane_max edges at most.) Measured on B200, 10 iterations of a settled vertex of 60000 edges beside
-// 60000 vertices that move in pairs: never pulled 0.36 ms, pulled whatever the list 6.95 ms. Every block reads the
-// same counter after the barrier, so all agree; the choice changes what the flags hold, not the result.
+// iteration it hold a quarter of the edges or more (the first iteration always does, pull_for), and no
+// list of region 1 that one warp would read to its end in vain is so long as to outlast the iteration: L
+// edges take L / 256 round trips of about half a microsecond, a balanced iteration m / 250 G/s, so L up to
+// m / 512. (Split vertices are searched by all their chunks' warps, hub_pull; the lists of smaller groups
+// are 16 * lane_max edges at most: the same rule for them made 4096 settled edges 0.73 -> 0.44 ms over 30
+// iterations, and the exact mode's kernel 2% slower.) Measured on B200, 30 iterations of a settled vertex of
+// 60000 edges beside vertices that move in pairs: never pulled 1.22 ms, pulled whatever the list 19.6 ms,
+// this 1.22 ms. Every block reads the same counter after the barrier, so all agree; the choice changes what
+// the flags hold, not the result.
 __device__ __forceinline__ bool pulls_next(const LpaArgs &a, int it, bool can_pull) {
   return can_pull && it + 2 < a.iters &&   // negative: LONG_IDLE
          (long long)__ldcg(a.stats + STATS_STRIDE * it + STAT_MOVED_EDGES) >= (a.m + 3) / 4;
